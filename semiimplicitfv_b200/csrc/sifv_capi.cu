@@ -20,6 +20,7 @@
 #include "sifv_kernels.cuh"
 #include "sifv_gs_march.cuh"
 #include "sifv_mg.cuh"
+#include "sifv_stage_api.h"
 #include "sifv_sweep_api.h"
 #include "sifv_ib_api.h"
 #include "sifv_vtk_api.h"
@@ -43,6 +44,8 @@ struct sifv_ctx {
     cudaStream_t stream = nullptr;
     cudaStream_t ownStream = nullptr;
     std::vector<void*> allocs;
+    char* arena = nullptr;     // the unused part of the last chunk (dalloc)
+    size_t arenaLeft = 0;
     Ctl* ctl = nullptr;        // device control block
     Ctl* ctlHost = nullptr;    // pinned mirror
     int resCap = 0;
@@ -98,8 +101,14 @@ struct sifv_ctx {
     bool uniformAxes = false;                 // interior cell widths bitwise equal along every active axis
     int pressureKind = 0;                     // 0 Jacobi (default), 1 Gauss-Seidel
     double* gsCoef = nullptr;                 // per-cell Gauss-Seidel coefficients (2 dim + 2 arrays)
-    double* tileB[4] = {nullptr, nullptr, nullptr, nullptr};   // 2D fused-stage scratch states
-    double* tileC[4] = {nullptr, nullptr, nullptr, nullptr};                // dynamic shared memory limit of the IGR tile kernel set
+    double* tileB[5] = {};                    // scratch states of the 2D fast and mixed stage kernel
+    double* tileC[5] = {};
+    StageState stageB{}, stageC{};            // scratch states of the fused stage kernel
+    bool stageReady = false;
+    bool splitReady = false;                  // step-start copies and face fluxes are allocated
+    bool advPending = false;                  // the previous step's time_advance is due (device-resident loops)
+    double* advLog = nullptr;
+    int advSlot = 0;
     double* lam[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     double* acc0[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     double* share[3] = {nullptr, nullptr, nullptr};
@@ -231,16 +240,29 @@ int validate(const sifv_config_t* c, std::string& msg) {
     return SIFV_OK;
 }
 
+// n zeroed doubles that live as long as the context, 256-byte aligned.  Small
+// arrays share chunks of up to eight (64 MB at most): a cudaMalloc costs a
+// few tenths of a millisecond, and a context holds 20 to 60 arrays.
 double* dalloc(sifv_ctx* c, size_t n, int& st) {
-    void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(double));
-    if (e != cudaSuccess) {
-        st = fail(c, SIFV_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-        return nullptr;
+    const size_t need = (std::max<size_t>(n, 1) * sizeof(double) + 255) / 256 * 256;
+    if (c->arenaLeft < need) {
+        const size_t chunk = std::max(need, std::min<size_t>(8 * need, (size_t)64 << 20));
+        void* p = nullptr;
+        cudaError_t e = cudaMalloc(&p, chunk);
+        if (e != cudaSuccess) {
+            st = fail(c, SIFV_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+            return nullptr;
+        }
+        c->allocs.push_back(p);
+        cudaMemsetAsync(p, 0, chunk, c->stream);
+        if (chunk - need < c->arenaLeft) return static_cast<double*>(p);   // keep the chunk with more room
+        c->arena = static_cast<char*>(p);
+        c->arenaLeft = chunk;
     }
-    cudaMemsetAsync(p, 0, std::max<size_t>(n, 1) * sizeof(double), c->stream);
-    c->allocs.push_back(p);
-    return static_cast<double*>(p);
+    double* r = reinterpret_cast<double*>(c->arena);
+    c->arena += need;
+    c->arenaLeft -= need;
+    return r;
 }
 
 double* field_ptr(sifv_ctx* c, int f) {
@@ -1363,6 +1385,62 @@ int reduce_residual(sifv_ctx* c, unsigned long long* slot) {
     return SIFV_OK;
 }
 
+// k_dt_finalize with programmatic dependent launch, closing the previous
+// step of a device-resident loop where that is due.
+int launch_dt_finalize(sifv_ctx* c, double constDt, double targetDt, int clampSemi, double minDt, double maxDt,
+                       int useEnd, double resetDt) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(1);
+    lc.blockDim = dim3(1);
+    lc.stream = c->stream;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    CUDA_TRY(c, cudaLaunchKernelEx(&lc, k_dt_finalize, c->ctl, constDt, targetDt, clampSemi, minDt, maxDt, useEnd,
+                                   resetDt, c->advPending ? 1 : 0, c->advLog, c->advSlot));
+    c->advPending = false;
+    c->launches++;
+    return SIFV_OK;
+}
+
+// The device-side dt log of a device-resident loop, at least n entries.
+int loop_log(sifv_ctx* c, int n) {
+    if (c->loopLogCap >= n) return SIFV_OK;
+    if (c->loopLog) cudaFree(c->loopLog);
+    c->loopLog = nullptr;
+    c->loopLogCap = 0;
+    CUDA_TRY(c, cudaMalloc(&c->loopLog, sizeof(double) * n));
+    c->loopLogCap = n;
+    return SIFV_OK;
+}
+
+// The last step of a device-resident loop: its time_advance, if still due.
+void flush_advance(sifv_ctx* c) {
+    if (!c->advPending) return;
+    k_time_advance<<<1, 1, 0, c->stream>>>(c->ctl, c->advLog, c->advSlot);
+    c->launches++;
+    c->advPending = false;
+}
+
+// The explicit steps that run as fused stage kernels (sifv_stage.cuh): the
+// reference-ordered mode in 1D and 2D with the five-cell stencils and at most
+// two phases, where nothing runs between the kernels of a stage (IGR, halo
+// exchange, immersed bodies, the adjoint's and tangent's hooks) and no
+// capillary stress is added.  One-stage schemes would need their output
+// copied back over their input and keep the separate kernels.
+bool fused_stage(const sifv_ctx* c) {
+    const Params& P = c->P;
+    return c->cfg.precision == SIFV_PREC_FP64 && !c->cfg.semiImplicit && !c->cfg.useIGR && P.dim <= 2 && c->W == 5 &&
+           c->nphT <= 2 && c->cfg.RKOrder > 1 && !P.cap && !c->ib.count && !c->F.solid && !c->exchangeFaces &&
+           !c->stageHook && P.ngx <= kStageMaxGhost && P.ny <= 8 * 65535;
+}
+
+// Whether the step's last stage folds the next step's dt limits into
+// ctl->dtBits.
+bool folds_dt(const sifv_ctx* c) { return (c->sweep && c->P.dim == 2) || fused_stage(c); }
+
 int enqueue_dt(sifv_ctx* c, double targetDt, int useEnd) {
     const sifv_config_t& cfg = c->cfg;
     unsigned g = blocks((long long)c->nint, kCellThreads);
@@ -1381,11 +1459,12 @@ int enqueue_dt(sifv_ctx* c, double targetDt, int useEnd) {
         if (c->comm.allreduce_min &&
             c->comm.allreduce_min(c->comm.user, reinterpret_cast<double*>(&c->ctl->dtBits), c->stream) != 0)
             return fail(c, SIFV_ERR_CUDA, "dt reduction over the ranks failed");
-        k_dt_finalize<<<1, 1, 0, c->stream>>>(c->ctl, -1.0, targetDt, 1, cfg.siMinDt, cfg.siMaxDt, useEnd);
-        c->launches += 3;
+        int st = launch_dt_finalize(c, -1.0, targetDt, 1, cfg.siMinDt, cfg.siMaxDt, useEnd, 0.0);
+        if (st != SIFV_OK) return st;
+        c->launches += 2;
     } else if (c->forcedDt > 0) {
-        k_dt_finalize<<<1, 1, 0, c->stream>>>(c->ctl, c->forcedDt, -1.0, 0, 0.0, 0.0, 0);
-        c->launches += 1;
+        int st = launch_dt_finalize(c, c->forcedDt, -1.0, 0, 0.0, 0.0, 0, 0.0);
+        if (st != SIFV_OK) return st;
     } else {
         if (cfg.constDt <= 0 && c->dtReady) {
             // the previous step's last stage left min(maxDt, acoustic dt) of this state in ctl->dtBits
@@ -1407,11 +1486,112 @@ int enqueue_dt(sifv_ctx* c, double targetDt, int useEnd) {
             c->comm.allreduce_min(c->comm.user, reinterpret_cast<double*>(&c->ctl->dtBits), c->stream) != 0)
             return fail(c, SIFV_ERR_CUDA, "dt reduction over the ranks failed");
         c->dtReady = false;
-        k_dt_finalize<<<1, 1, 0, c->stream>>>(c->ctl, cfg.constDt, targetDt, 0, 0.0, 0.0, useEnd);
-        c->launches += 1;
+        int st = launch_dt_finalize(c, cfg.constDt, targetDt, 0, 0.0, 0.0, useEnd,
+                                    (cfg.constDt <= 0 && folds_dt(c)) ? cfg.maxDt : 0.0);
+        if (st != SIFV_OK) return st;
     }
     mark(c, "dt");
     return SIFV_OK;
+}
+
+// The context's state, and two scratch states of its shape, for the fused
+// stage kernel.
+StageState stage_state(const sifv_ctx* c) {
+    const Fields& F = c->F;
+    StageState S{};
+    S.rho = F.rho;
+    S.mom[0] = F.rhoU;
+    S.mom[1] = F.rhoV;
+    S.mom[2] = F.rhoW;
+    S.rhoE = F.rhoE;
+    for (int ph = 0; ph < c->P.nPh && ph < 2; ++ph) {
+        S.alphaRho[ph] = F.alphaRho[ph];
+        S.alpha[ph] = F.alpha[ph];
+    }
+    return S;
+}
+
+// Step-start copies and face fluxes of the separate stage kernels, allocated
+// with the context, or on the first step that needs them where the fused
+// stage kernel runs instead (a context that later gets immersed bodies, or a
+// tangent run).
+int split_buffers(sifv_ctx* c) {
+    if (c->splitReady) return SIFV_OK;
+    const sifv_config_t* cfg = &c->cfg;
+    const Params& P = c->P;
+    Fields& F = c->F;
+    const int dim = P.dim, nx = P.nx, ny = P.ny, nz = P.nz;
+    const size_t n = c->ncells;
+    int st = SIFV_OK;
+    if (cfg->RKOrder > 1) {
+        F.rho0 = dalloc(c, n, st); F.rhoU0 = dalloc(c, n, st); F.rhoE0 = dalloc(c, n, st); F.pres0 = dalloc(c, n, st);
+        if (dim >= 2) F.rhoV0 = dalloc(c, n, st);
+        if (dim >= 3) F.rhoW0 = dalloc(c, n, st);
+        for (int p = 0; p < cfg->nPhases; ++p) { F.alphaRho0[p] = dalloc(c, n, st); F.alpha0[p] = dalloc(c, n, st); }
+    }
+    for (int d = 0; d < dim && !c->sweep; ++d) {   // the dimension sweeps keep no face arrays
+        size_t nf = (size_t)(nx + (d == 0)) * (ny + (d == 1)) * (nz + (d == 2));
+        F.flux[d][FS_MASS] = dalloc(c, nf, st);
+        F.flux[d][FS_MOMX] = dalloc(c, nf, st);
+        if (dim >= 2) F.flux[d][FS_MOMY] = dalloc(c, nf, st);
+        if (dim >= 3) F.flux[d][FS_MOMZ] = dalloc(c, nf, st);
+        F.flux[d][FS_ENERGY] = dalloc(c, nf, st);
+        if (cfg->semiImplicit) F.flux[d][FS_PFLUX] = dalloc(c, nf, st);
+        if (cfg->semiImplicit || cfg->nPhases > 0) F.flux[d][FS_FVEL] = dalloc(c, nf, st);
+        for (int p = 0; p < cfg->nPhases; ++p) {
+            F.flux[d][FS_ALPHA + p] = dalloc(c, nf, st);
+            F.flux[d][FS_AR + p] = dalloc(c, nf, st);
+        }
+        if (P.visc)
+            for (int q = 0; q < 4; ++q) F.flux[d][FS_VISC + q] = (q == 0 || q == 3 || q < dim) ? dalloc(c, nf, st) : nullptr;
+        if (P.cap)
+            for (int q = 0; q < 4; ++q) F.flux[d][FS_CAP + q] = (q == 0 || q == 3 || q < dim) ? dalloc(c, nf, st) : nullptr;
+    }
+    c->splitReady = st == SIFV_OK;
+    return st;
+}
+
+// Scratch states of the 2D fast / mixed stage kernel.
+int tile_buffers(sifv_ctx* c) {
+    int st = SIFV_OK;
+    for (int q = 0; q < c->P.dim + 2; ++q) {
+        c->tileB[q] = dalloc(c, c->ncells, st);
+        c->tileC[q] = dalloc(c, c->ncells, st);
+    }
+    return st;
+}
+
+int stage_buffers(sifv_ctx* c) {
+    if (c->stageReady) return SIFV_OK;
+    int st = SIFV_OK;
+    for (StageState* S : {&c->stageB, &c->stageC}) {
+        S->rho = dalloc(c, c->ncells, st);
+        for (int d = 0; d < c->P.dim; ++d) S->mom[d] = dalloc(c, c->ncells, st);
+        S->rhoE = dalloc(c, c->ncells, st);
+        for (int ph = 0; ph < c->P.nPh; ++ph) {
+            S->alphaRho[ph] = dalloc(c, c->ncells, st);
+            S->alpha[ph] = dalloc(c, c->ncells, st);
+        }
+    }
+    c->stageReady = st == SIFV_OK;
+    return st;
+}
+
+// Everything of stage s but the states and the last stage's switches.
+StageArgs stage_args(const sifv_ctx* c, int s) {
+    StageArgs A{};
+    A.P = c->P;
+    A.ctl = c->ctl;
+    rk_coef(c->cfg.RKOrder, s, A.K);
+    A.cfl = c->cfg.cfl;
+    A.velU = c->F.velU;
+    A.velV = c->F.velV;
+    A.pres = c->F.pres;
+    A.sigma = c->F.sigma;
+    A.dx = c->F.dx;
+    A.dy = c->F.dy;
+    A.dz = c->F.dz;
+    return A;
 }
 
 // One step, everything enqueued on the stream; semi-implicit steps
@@ -1428,14 +1608,6 @@ int enqueue_step(sifv_ctx* c, int step, double time, double targetDt, int useEnd
     if (c->sweep && P.dim == 2) {
         // one fused tile kernel per stage; stage outputs ping-pong through two
         // scratch states, the last stage writes over the step-start state
-        if (!c->tileB[0]) {
-            int sa = SIFV_OK;
-            for (int q = 0; q < 4; ++q) {
-                c->tileB[q] = dalloc(c, c->ncells, sa);
-                c->tileC[q] = dalloc(c, c->ncells, sa);
-            }
-            if (sa != SIFV_OK) return sa;
-        }
         double* U[4] = {c->F.rho, c->F.rhoU, c->F.rhoV, c->F.rhoE};
         const int RK = cfg.RKOrder;
         for (int s = 0; s < RK; ++s) {
@@ -1459,10 +1631,6 @@ int enqueue_step(sifv_ctx* c, int step, double time, double targetDt, int useEnd
             T.cfl = cfg.cfl;
             T.dx = c->F.dx;
             T.dy = c->F.dy;
-            if (T.dtNext) {   // accumulator of the next step's dt
-                k_dt_init<<<1, 1, 0, c->stream>>>(c->ctl, cfg.maxDt);
-                c->launches++;
-            }
             T.velU = c->F.velU;
             T.velV = c->F.velV;
             T.pres = c->F.pres;
@@ -1524,6 +1692,31 @@ int enqueue_step(sifv_ctx* c, int step, double time, double targetDt, int useEnd
         launch_bc_prim(c);
         LAUNCH_CHECK(c);
         return SIFV_OK;
+    }
+    if (fused_stage(c)) {
+        int st = stage_buffers(c);
+        if (st != SIFV_OK) return st;
+        const int RK = cfg.RKOrder;
+        const bool fold = cfg.constDt <= 0 && c->forcedDt <= 0;
+        for (int s = 0; s < RK; ++s) {
+            StageArgs A = stage_args(c, s);
+            body_force(cfg, time, A.K);
+            A.u0 = stage_state(c);
+            A.in = (s == 0) ? A.u0 : (s == 1) ? c->stageB : c->stageC;
+            A.out = (s == RK - 1) ? A.u0 : (s == 0) ? c->stageB : c->stageC;
+            A.last = (s == RK - 1) ? 1 : 0;
+            A.dtNext = (A.last && fold) ? 1 : 0;
+            if (stage_launch(A, c->stream) != 0) return fail(c, SIFV_ERR_CUDA, "stage launch failed");
+            c->launches++;
+            mark(c, "stage");
+        }
+        LAUNCH_CHECK(c);
+        c->dtReady = fold;
+        return SIFV_OK;
+    }
+    {
+        int st = split_buffers(c);
+        if (st != SIFV_OK) return st;
     }
     for (int s = 0; s < cfg.RKOrder; ++s) {
         StageCoef K{};
@@ -1767,12 +1960,6 @@ int sifv_create(const sifv_config_t* cfg, const sifv_mesh_t* mesh, int device, s
     if (dim >= 2) { F.rhoV = dalloc(c, n, st); F.velV = dalloc(c, n, st); }
     if (dim >= 3) { F.rhoW = dalloc(c, n, st); F.velW = dalloc(c, n, st); }
     for (int p = 0; p < cfg->nPhases; ++p) { F.alphaRho[p] = dalloc(c, n, st); F.alpha[p] = dalloc(c, n, st); }
-    if (cfg->RKOrder > 1) {
-        F.rho0 = dalloc(c, n, st); F.rhoU0 = dalloc(c, n, st); F.rhoE0 = dalloc(c, n, st); F.pres0 = dalloc(c, n, st);
-        if (dim >= 2) F.rhoV0 = dalloc(c, n, st);
-        if (dim >= 3) F.rhoW0 = dalloc(c, n, st);
-        for (int p = 0; p < cfg->nPhases; ++p) { F.alphaRho0[p] = dalloc(c, n, st); F.alpha0[p] = dalloc(c, n, st); }
-    }
     if (cfg->semiImplicit) {
         F.rhoUStar = dalloc(c, n, st); F.rhoEstar = dalloc(c, n, st); F.pAdvected = dalloc(c, n, st);
         F.rhoc2 = dalloc(c, n, st);
@@ -1782,24 +1969,6 @@ int sifv_create(const sifv_config_t* cfg, const sifv_mesh_t* mesh, int device, s
     }
     F.pA = dalloc(c, n, st); F.pB = dalloc(c, n, st);
     if (cfg->useIGR) { F.igrRhs = dalloc(c, n, st); F.igrDiag = dalloc(c, n, st); }
-    for (int d = 0; d < dim; ++d) {
-        size_t nf = (size_t)(nx + (d == 0)) * (ny + (d == 1)) * (nz + (d == 2));
-        F.flux[d][FS_MASS] = dalloc(c, nf, st);
-        F.flux[d][FS_MOMX] = dalloc(c, nf, st);
-        if (dim >= 2) F.flux[d][FS_MOMY] = dalloc(c, nf, st);
-        if (dim >= 3) F.flux[d][FS_MOMZ] = dalloc(c, nf, st);
-        F.flux[d][FS_ENERGY] = dalloc(c, nf, st);
-        if (cfg->semiImplicit) F.flux[d][FS_PFLUX] = dalloc(c, nf, st);
-        if (cfg->semiImplicit || cfg->nPhases > 0) F.flux[d][FS_FVEL] = dalloc(c, nf, st);
-        for (int p = 0; p < cfg->nPhases; ++p) {
-            F.flux[d][FS_ALPHA + p] = dalloc(c, nf, st);
-            F.flux[d][FS_AR + p] = dalloc(c, nf, st);
-        }
-        if (P.visc)
-            for (int q = 0; q < 4; ++q) F.flux[d][FS_VISC + q] = (q == 0 || q == 3 || q < dim) ? dalloc(c, nf, st) : nullptr;
-        if (P.cap)
-            for (int q = 0; q < 4; ++q) F.flux[d][FS_CAP + q] = (q == 0 || q == 3 || q < dim) ? dalloc(c, nf, st) : nullptr;
-    }
     // geometry: per-cell widths incl. ghosts, and IGR alpha/d^2
     static const double unit[2] = {0.0, 1.0};
     std::vector<double> xe = build_ext(mesh->xNodes, nx, P.ngx);
@@ -1862,6 +2031,7 @@ int sifv_create(const sifv_config_t* cfg, const sifv_mesh_t* mesh, int device, s
         if (st == SIFV_OK) cudaStreamSynchronize(c->stream);   // host vectors above go out of scope
     }
     if (st == SIFV_OK) st = ensure_res(c, std::max(cfg->maxPressureIters, 1));
+    if (st == SIFV_OK) st = fused_stage(c) ? stage_buffers(c) : (c->sweep && dim == 2) ? tile_buffers(c) : split_buffers(c);
     if (st == SIFV_OK) {
         cudaError_t e = cudaStreamSynchronize(c->stream);
         if (e != cudaSuccess) st = fail(c, SIFV_ERR_CUDA, cudaGetErrorString(e));
@@ -1912,14 +2082,6 @@ int sifv_autotune(sifv_ctx_t* c, int reps, int* choice) {
     *choice = 0;
     if (!(c->sweep && c->P.dim == 2)) return SIFV_OK;   // only the 2D fused stage has a shape to tune
     cudaSetDevice(c->device);
-    if (!c->tileB[0]) {
-        int sa = SIFV_OK;
-        for (int q = 0; q < 4; ++q) {
-            c->tileB[q] = dalloc(c, c->ncells, sa);
-            c->tileC[q] = dalloc(c, c->ncells, sa);
-        }
-        if (sa != SIFV_OK) return sa;
-    }
     // probe: the first stage of a step from the current state into the scratch
     // state (the state itself is not written), no primitives, no dt
     const sifv_config_t& cfg = c->cfg;
@@ -2048,10 +2210,15 @@ int sifv_advance(sifv_ctx_t* c, int step0, double time0, double tEnd, int nSteps
     int status = SIFV_OK;
     for (int q = 0; q < nSteps; ++q) {
         int st = enqueue_step(c, step0 + q, time0, -1.0, true, status);
-        if (st != SIFV_OK) return st;
-        k_time_advance<<<1, 1, 0, c->stream>>>(c->ctl);
-        c->launches++;
+        if (st != SIFV_OK) {
+            c->advPending = false;
+            return st;
+        }
+        c->advPending = true;
+        c->advLog = nullptr;
+        c->advSlot = 0;
     }
+    flush_advance(c);
     CUDA_TRY(c, cudaEventRecord(c->ev1, c->stream));
     CUDA_TRY(c, cudaMemcpyAsync(c->ctlHost, c->ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
@@ -2366,6 +2533,7 @@ int run_forward(sifv_ctx* c, int step0, double time0, double tEnd, int maxSteps,
                 int every, bool record, double& timeOut, int& stepsOut) {
     double t = time0;
     int q = 0;
+    c->dtReady = false;   // the state may have changed since the last call
     for (;;) {
         if (sched) {
             if (q >= nSched) break;
@@ -2863,13 +3031,8 @@ int sifv_run_time_loop(sifv_ctx_t* c, const sifv_time_loop_t* prm, sifv_vtk_t* v
         return finish(SIFV_OK);
     }
     const int batchMax = prm->batch > 0 ? prm->batch : 64;
-    if (c->loopLogCap < batchMax) {
-        if (c->loopLog) cudaFree(c->loopLog);
-        c->loopLog = nullptr;
-        c->loopLogCap = 0;
-        CUDA_TRY(c, cudaMalloc(&c->loopLog, sizeof(double) * batchMax));
-        c->loopLogCap = batchMax;
-    }
+    st = loop_log(c, batchMax);
+    if (st != SIFV_OK) return finish(st);
     std::vector<double> log(batchMax);
     Ctl h{};
     h.time = 0.0;
@@ -2884,10 +3047,15 @@ int sifv_run_time_loop(sifv_ctx_t* c, const sifv_time_loop_t* prm, sifv_vtk_t* v
         int status = SIFV_OK;
         for (int q = 0; q < B; ++q) {
             st = enqueue_step(c, step + q, 0.0, -1.0, 2, status);
-            if (st != SIFV_OK) return finish(st);
-            k_time_advance<<<1, 1, 0, c->stream>>>(c->ctl, c->loopLog, q);
-            c->launches++;
+            if (st != SIFV_OK) {
+                c->advPending = false;
+                return finish(st);
+            }
+            c->advPending = true;
+            c->advLog = c->loopLog;
+            c->advSlot = q;
         }
+        flush_advance(c);
         LAUNCH_CHECK(c);
         CUDA_TRY(c, cudaMemcpyAsync(c->ctlHost, c->ctl, offsetof(Ctl, res), cudaMemcpyDeviceToHost, c->stream));
         CUDA_TRY(c, cudaMemcpyAsync(log.data(), c->loopLog, sizeof(double) * B, cudaMemcpyDeviceToHost, c->stream));

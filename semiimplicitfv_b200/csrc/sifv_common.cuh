@@ -11,6 +11,11 @@ namespace sifv {
 __device__ __forceinline__ double bits2d(unsigned long long b) { return __longlong_as_double((long long)b); }
 __device__ __forceinline__ unsigned long long d2bits(double d) { return (unsigned long long)__double_as_longlong(d); }
 
+// Programmatic dependent launch: let the next kernel of the stream be set up
+// now; wait for the previous one (both no-ops on an ordinary launch).
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
 // Split a linear id t = a + n0 (b + n1 c) into (a, b, c); 32-bit unsigned
 // division when t fits (every grid up to 2^32 cells), 64-bit otherwise.
 __device__ __forceinline__ void split3(long long t, int n0, int n1, int& a, int& b, int& c) {
@@ -180,6 +185,76 @@ __device__ __forceinline__ void cell_faces(const Params& P, const Fields& F, int
     cf.hiOff[1] = P.nx;
     cf.lo[2] = (long long)i + (long long)P.nx * ((long long)j + (long long)P.ny * k);
     cf.hiOff[2] = (long long)P.nx * P.ny;
+}
+
+// Viscous stress on one face of direction DIR (src/ViscousFlux.cpp:24-303):
+// normal gradients over the two cells' width, transverse central differences
+// averaged over the two cells, the divergence, and the work with the
+// face-averaged velocity.  U, V, W are indexed by I with strides sx, sy, sz;
+// iL, iR are the cells left and right of the face; px, py, pz point at the
+// widths of the right cell (the left cell's are at [-1] along DIR).
+template <int DIR, typename I>
+__device__ __forceinline__ void visc_stress(int dim, const double* U, const double* V, const double* W, I iL, I iR,
+                                            I sx, I sy, I sz, const double* px, const double* py, const double* pz,
+                                            double muF, double tau[3], double& work) {
+    double uF, vF = 0.0, wF = 0.0;
+    // average over the two cells of the central difference of q along a transverse axis
+    auto cross = [&](const double* q, I st, double d) {
+        double gL = (q[iL + st] - q[iL - st]) / (2.0 * d), gR = (q[iR + st] - q[iR - st]) / (2.0 * d);
+        return 0.5 * (gL + gR);
+    };
+    if (DIR == 0) {
+        double dxi = 0.5 * (px[-1] + px[0]);
+        double dudx = (U[iR] - U[iL]) / dxi, dvdx = 0.0, dwdx = 0.0;
+        if (dim >= 2) dvdx = (V[iR] - V[iL]) / dxi;
+        if (dim >= 3) dwdx = (W[iR] - W[iL]) / dxi;
+        double dudy = 0.0, dvdy = 0.0, dudz = 0.0, dwdz = 0.0;
+        if (dim >= 2) {
+            dudy = cross(U, sy, py[0]);
+            dvdy = cross(V, sy, py[0]);
+        }
+        if (dim >= 3) {
+            dudz = cross(U, sz, pz[0]);
+            dwdz = cross(W, sz, pz[0]);
+        }
+        double divU = dudx + dvdy + dwdz;
+        tau[0] = muF * (2.0 * dudx - (2.0 / 3.0) * divU);
+        tau[1] = muF * (dvdx + dudy);
+        tau[2] = muF * (dwdx + dudz);
+        uF = 0.5 * (U[iL] + U[iR]);
+        if (dim >= 2) vF = 0.5 * (V[iL] + V[iR]);
+        if (dim >= 3) wF = 0.5 * (W[iL] + W[iR]);
+    } else if (DIR == 1) {
+        double dyj = 0.5 * (py[-1] + py[0]);
+        double dudy = (U[iR] - U[iL]) / dyj, dvdy = (V[iR] - V[iL]) / dyj, dwdy = 0.0;
+        if (dim >= 3) dwdy = (W[iR] - W[iL]) / dyj;
+        double dudx = cross(U, sx, px[0]), dvdx = cross(V, sx, px[0]);
+        double dvdz = 0.0, dwdz = 0.0;
+        if (dim >= 3) {
+            dvdz = cross(V, sz, pz[0]);
+            dwdz = cross(W, sz, pz[0]);
+        }
+        double divU = dudx + dvdy + dwdz;
+        tau[0] = muF * (dudy + dvdx);
+        tau[1] = muF * (2.0 * dvdy - (2.0 / 3.0) * divU);
+        tau[2] = muF * (dwdy + dvdz);
+        uF = 0.5 * (U[iL] + U[iR]);
+        vF = 0.5 * (V[iL] + V[iR]);
+        if (dim >= 3) wF = 0.5 * (W[iL] + W[iR]);
+    } else {
+        double dzk = 0.5 * (pz[-1] + pz[0]);
+        double dudz = (U[iR] - U[iL]) / dzk, dvdz = (V[iR] - V[iL]) / dzk, dwdz = (W[iR] - W[iL]) / dzk;
+        double dudx = cross(U, sx, px[0]), dwdx = cross(W, sx, px[0]);
+        double dvdy = cross(V, sy, py[0]), dwdy = cross(W, sy, py[0]);
+        double divU = dudx + dvdy + dwdz;
+        tau[0] = muF * (dudz + dwdx);
+        tau[1] = muF * (dvdz + dwdy);
+        tau[2] = muF * (2.0 * dwdz - (2.0 / 3.0) * divU);
+        uF = 0.5 * (U[iL] + U[iR]);
+        vF = 0.5 * (V[iL] + V[iR]);
+        wF = 0.5 * (W[iL] + W[iR]);
+    }
+    work = tau[0] * uF + tau[1] * vF + tau[2] * wF;
 }
 
 // Block-wide minimum of non-negative doubles, NaN ignored (std::min(dt, x)

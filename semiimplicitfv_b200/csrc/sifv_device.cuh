@@ -17,6 +17,7 @@
 #include <cstdint>
 
 #include "sifv.h"
+#include "sifv_rn.cuh"
 
 // Loop over the active axes 0..dim-1, unrolled to 3 with a uniform guard so
 // per-axis arrays stay in registers.
@@ -292,6 +293,54 @@ __device__ __forceinline__ T weno5R(T v0, T v1, T v2, T v3, T v4, T eps) {
     return (a0 * p0 + a1 * p1 + a2 * p2) / aSum;
 }
 
+// weno5L in the reference's order with every division as a branch-free
+// correctly rounded quotient (sifv_rn.cuh); bit-identical to weno5L.  The
+// mirrored call weno5_rn(v4, v3, v2, v1, v0) is weno5R(v0, .., v4).  2 v and
+// 4 v are exact, so their products ride in fused multiply-adds, and so does
+// the quarter of a square (the difference, below 2^-1022, vanishes against
+// eps).  Smoothness indicators above 2^256, an eps outside [1e-100, 1e100]
+// and final operands outside div_markstein's range take weno5_plain.
+// 98 + 8 x 8 FP64 operations for two sides of a cell against 108 + 8
+// divisions.
+static __device__ __noinline__ double weno5_plain(double v0, double v1, double v2, double v3, double v4, double eps) {
+    return weno5L<double>(v0, v1, v2, v3, v4, eps);
+}
+__device__ __forceinline__ double weno5_rn(double v0, double v1, double v2, double v3, double v4, double eps) {
+    const double p0 = (1.0 / 3.0) * v0 - (7.0 / 6.0) * v1 + (11.0 / 6.0) * v2;
+    const double p1 = -(1.0 / 6.0) * v1 + (5.0 / 6.0) * v2 + (1.0 / 3.0) * v3;
+    const double p2 = (1.0 / 3.0) * v2 + (5.0 / 6.0) * v3 - (1.0 / 6.0) * v4;
+    const double t0 = fma(-2.0, v1, v0) + v2, s0 = fma(-4.0, v1, v0) + 3.0 * v2;
+    const double t1 = fma(-2.0, v2, v1) + v3, s1 = v1 - v3;
+    const double t2 = fma(-2.0, v3, v2) + v4, s2 = fma(-4.0, v3, 3.0 * v2) + v4;
+    const double e0 = eps + fma(0.25, s0 * s0, (13.0 / 12.0) * t0 * t0);
+    const double e1 = eps + fma(0.25, s1 * s1, (13.0 / 12.0) * t1 * t1);
+    const double e2 = eps + fma(0.25, s2 * s2, (13.0 / 12.0) * t2 * t2);
+    const double E0 = e0 * e0, E1 = e1 * e1, E2 = e2 * e2;
+    const double a0 = div_weight_rn(1.0 / 10.0, E0, rcp_near(E0));
+    const double a1 = div_weight_rn(6.0 / 10.0, E1, rcp_near(E1));
+    const double a2 = div_weight_rn(3.0 / 10.0, E2, rcp_near(E2));
+    const double aSum = a0 + a1 + a2;
+    const double num = a0 * p0 + a1 * p1 + a2 * p2;
+    const double q = div_markstein(num, aSum, rcp_rn(aSum, rcp_near(aSum)));
+    // positive numbers (or NaN) compare as integers: every E below 2^513
+    const unsigned hi = max(max((unsigned)__double2hiint(E0), (unsigned)__double2hiint(E1)), (unsigned)__double2hiint(E2));
+    const bool fine = hi < 0x60000000u && rn_fast_operand(num) && rn_fast_recip(aSum) &&
+                      __double2loint(aSum) != -1 && eps >= 1e-100 && eps <= 1e100;
+    return fine ? q : weno5_plain(v0, v1, v2, v3, v4, eps);
+}
+template <typename T>
+__device__ __forceinline__ T weno5_high(T v0, T v1, T v2, T v3, T v4, T eps) { return weno5L<T>(v0, v1, v2, v3, v4, eps); }
+template <typename T>
+__device__ __forceinline__ T weno5_low(T v0, T v1, T v2, T v3, T v4, T eps) { return weno5R<T>(v0, v1, v2, v3, v4, eps); }
+template <>
+__device__ __forceinline__ double weno5_high(double v0, double v1, double v2, double v3, double v4, double eps) {
+    return weno5_rn(v0, v1, v2, v3, v4, eps);
+}
+template <>
+__device__ __forceinline__ double weno5_low(double v0, double v1, double v2, double v3, double v4, double eps) {
+    return weno5_rn(v4, v3, v2, v1, v0, eps);
+}
+
 template <typename T>
 __device__ __forceinline__ T upwind5L(T v0, T v1, T v2, T v3, T v4) {
     T p0 = (T(1.0) / T(3.0)) * v0 - (T(7.0) / T(6.0)) * v1 + (T(11.0) / T(6.0)) * v2;
@@ -371,8 +420,8 @@ __device__ __forceinline__ void recon_pair(const T* __restrict__ f, size_t base,
         T v0 = f[base - 3 * st], v1 = f[base - 2 * st], v2 = f[base - st], v3 = f[base], v4 = f[base + st],
                v5 = f[base + 2 * st];
         if (weno) {
-            L = weno5L(v0, v1, v2, v3, v4, eps);
-            R = weno5R(v1, v2, v3, v4, v5, eps);
+            L = weno5_high(v0, v1, v2, v3, v4, eps);
+            R = weno5_low(v1, v2, v3, v4, v5, eps);
         } else {
             L = upwind5L(v0, v1, v2, v3, v4);
             R = upwind5R(v1, v2, v3, v4, v5);

@@ -1,7 +1,7 @@
 // sifv_gs_march.cuh -- 2D Gauss-Seidel iterations as one persistent
 // wavefront (GaussSeidelPressureSolver::solve, src/GaussSeidelPressureSolver.cpp:60-100,
 // on a 2D mesh without halo exchange).  Included by sifv_capi.cu after
-// sifv_kernels.cuh (gs_cell's arithmetic, div_markstein, igr_fast_*).
+// sifv_kernels.cuh (gs_cell's arithmetic, div_markstein, rn_fast_*).
 //
 // The lexicographic sweep (x fastest) computes cell (x, j) from the new
 // values at (x-1, j), (x, j-1) and the old ones at (x+1, j), (x, j+1), so
@@ -153,7 +153,7 @@ __device__ __forceinline__ double march_cell(bool act, bool fastRecs, double2 c0
     od += c1.x * ym + c1.y * yp;
     const double num = act ? c3.y + c2.x * od : 1.0;
     const double dv = act ? c2.y : 1.0, rdv = act ? c3.x : 1.0;
-    return (fastRecs && igr_fast_operand(num)) ? div_markstein(num, dv, rdv) : div_rn_plain(num, dv);
+    return (fastRecs && rn_fast_operand(num)) ? div_markstein(num, dv, rdv) : div_rn_plain(num, dv);
 }
 
 // The IGR update of one cell (igr_cell, src/IGR.cpp:110-156, 2D) from its
@@ -177,13 +177,13 @@ __device__ __forceinline__ double igr_march_cell(bool act, bool fastRecs, const 
                                                  double pR, double pD, double pU) {
     const double sxm = TR ? pD : pL, sxp = TR ? pU : pR, sym = TR ? pL : pD, syp = TR ? pR : pU;
     const double ax = TR ? wn : r[4].x, ay = TR ? r[4].x : wn;
-    if (!act || (fastRecs && igr_fast_operand(sxm) && igr_fast_operand(sxp) && igr_fast_operand(sym) &&
-                 igr_fast_operand(syp))) {
+    if (!act || (fastRecs && rn_fast_operand(sxm) && rn_fast_operand(sxp) && rn_fast_operand(sym) &&
+                 rn_fast_operand(syp))) {
         double off = 0.0;
         off += ax * (div_markstein(sxm, r[0].x, r[0].y) + div_markstein(sxp, r[1].x, r[1].y));
         off += ay * (div_markstein(sym, r[2].x, r[2].y) + div_markstein(syp, r[3].x, r[3].y));
         const double num = r[4].y + off;
-        return (!act || igr_fast_operand(num)) ? div_markstein(num, r[5].x, r[5].y) : div_rn_plain(num, r[5].x);
+        return (!act || rn_fast_operand(num)) ? div_markstein(num, r[5].x, r[5].y) : div_rn_plain(num, r[5].x);
     }
     return igr_cell_plain2(sxm, sxp, sym, syp, r[0].x, r[1].x, r[2].x, r[3].x, ax, ay, r[4].y, r[5].x);
 }
@@ -224,8 +224,8 @@ __global__ void k_march_igr_setup(Params P, Fields F, double2* __restrict__ rec,
             o[96] = make_double2(rfry, ryr);
             o[128] = make_double2(tr ? F.ady2[j + P.ngy] : F.adx2[i + P.ngx], F.igrRhs[c]);
             o[160] = make_double2(diag, rd);
-            if (!(igr_fast_recip(rxl) && igr_fast_recip(rxr) && igr_fast_recip(ryl) && igr_fast_recip(ryr) &&
-                  igr_fast_recip(rd)))
+            if (!(rn_fast_recip(rxl) && rn_fast_recip(rxr) && rn_fast_recip(ryl) && rn_fast_recip(ryr) &&
+                  rn_fast_recip(rd)))
                 atomicOr(slowRecs, 1);
         }
     }
@@ -257,7 +257,7 @@ __global__ void k_march_gs_setup(Params P, const double* __restrict__ coef, size
             o[32] = make_double2(coef[2 * nc + c], coef[3 * nc + c]);
             o[64] = make_double2(coef[4 * nc + c], denom);
             o[96] = make_double2(rd, rhs[c]);
-            if (!igr_fast_recip(rd)) atomicOr(slowRecs, 1);
+            if (!rn_fast_recip(rd)) atomicOr(slowRecs, 1);
         }
     }
     q0[id] = make_double2(v[0], v[1]);

@@ -473,12 +473,9 @@ __global__ void __launch_bounds__(256) k_visc_face(Params P, Fields F, const Ctl
     if (t >= tot) return;
     int i, j, k;
     split3(t, fnx, fny, i, j, k);
-    const double* U = F.velU;
-    const double* V = F.velV;
-    const double* W = F.velW;
-    auto at = [&](int a, int b, int c) { return cidx(P, a, b, c); };
-    const int li = i - (DIR == 0), lj = j - (DIR == 1), lk = k - (DIR == 2);
-    const size_t iL = at(li, lj, lk), iR = at(i, j, k);
+    const size_t iR = cidx(P, i, j, k);
+    const size_t sy = (size_t)P.nxT, sz = (size_t)P.nxT * P.nyT;
+    const size_t iL = iR - ((DIR == 0) ? 1 : (DIR == 1) ? sy : sz);
     double muF;
     if (!P.perPhaseMu) {
         muF = P.mu;
@@ -490,90 +487,13 @@ __global__ void __launch_bounds__(256) k_visc_face(Params P, Fields F, const Ctl
         }
         muF = 0.5 * (muL + muR);
     }
-    double t0, t1, t2, work;
-    if (DIR == 0) {
-        double dxi = 0.5 * (F.dx[i - 1 + P.ngx] + F.dx[i + P.ngx]);
-        double dudx = (U[iR] - U[iL]) / dxi, dvdx = 0.0, dwdx = 0.0;
-        if (dim >= 2) dvdx = (V[iR] - V[iL]) / dxi;
-        if (dim >= 3) dwdx = (W[iR] - W[iL]) / dxi;
-        double dudy = 0.0, dvdy = 0.0;
-        if (dim >= 2) {
-            double dyj = F.dy[j + P.ngy];
-            size_t Ljm = at(i - 1, j - 1, k), Ljp = at(i - 1, j + 1, k), Rjm = at(i, j - 1, k), Rjp = at(i, j + 1, k);
-            double dudyL = (U[Ljp] - U[Ljm]) / (2.0 * dyj), dudyR = (U[Rjp] - U[Rjm]) / (2.0 * dyj);
-            dudy = 0.5 * (dudyL + dudyR);
-            double dvdyL = (V[Ljp] - V[Ljm]) / (2.0 * dyj), dvdyR = (V[Rjp] - V[Rjm]) / (2.0 * dyj);
-            dvdy = 0.5 * (dvdyL + dvdyR);
-        }
-        double dudz = 0.0, dwdz = 0.0;
-        if (dim >= 3) {
-            double dzk = F.dz[k + P.ngz];
-            size_t Lkm = at(i - 1, j, k - 1), Lkp = at(i - 1, j, k + 1), Rkm = at(i, j, k - 1), Rkp = at(i, j, k + 1);
-            double dudzL = (U[Lkp] - U[Lkm]) / (2.0 * dzk), dudzR = (U[Rkp] - U[Rkm]) / (2.0 * dzk);
-            dudz = 0.5 * (dudzL + dudzR);
-            double dwdzL = (W[Lkp] - W[Lkm]) / (2.0 * dzk), dwdzR = (W[Rkp] - W[Rkm]) / (2.0 * dzk);
-            dwdz = 0.5 * (dwdzL + dwdzR);
-        }
-        double divU = dudx + dvdy + dwdz;
-        t0 = muF * (2.0 * dudx - (2.0 / 3.0) * divU);
-        t1 = muF * (dvdx + dudy);
-        t2 = muF * (dwdx + dudz);
-        double uF = 0.5 * (U[iL] + U[iR]), vF = 0.0, wF = 0.0;
-        if (dim >= 2) vF = 0.5 * (V[iL] + V[iR]);
-        if (dim >= 3) wF = 0.5 * (W[iL] + W[iR]);
-        work = t0 * uF + t1 * vF + t2 * wF;
-    } else if (DIR == 1) {
-        double dyj = 0.5 * (F.dy[j - 1 + P.ngy] + F.dy[j + P.ngy]);
-        double dudy = (U[iR] - U[iL]) / dyj, dvdy = (V[iR] - V[iL]) / dyj, dwdy = 0.0;
-        if (dim >= 3) dwdy = (W[iR] - W[iL]) / dyj;
-        double dxi = F.dx[i + P.ngx];
-        size_t Lim = at(i - 1, j - 1, k), Lip = at(i + 1, j - 1, k), Rim = at(i - 1, j, k), Rip = at(i + 1, j, k);
-        double dudxL = (U[Lip] - U[Lim]) / (2.0 * dxi), dudxR = (U[Rip] - U[Rim]) / (2.0 * dxi);
-        double dudx = 0.5 * (dudxL + dudxR);
-        double dvdxL = (V[Lip] - V[Lim]) / (2.0 * dxi), dvdxR = (V[Rip] - V[Rim]) / (2.0 * dxi);
-        double dvdx = 0.5 * (dvdxL + dvdxR);
-        double dvdz = 0.0, dwdz = 0.0;
-        if (dim >= 3) {
-            double dzk = F.dz[k + P.ngz];
-            size_t Lkm = at(i, j - 1, k - 1), Lkp = at(i, j - 1, k + 1), Rkm = at(i, j, k - 1), Rkp = at(i, j, k + 1);
-            double dvdzL = (V[Lkp] - V[Lkm]) / (2.0 * dzk), dvdzR = (V[Rkp] - V[Rkm]) / (2.0 * dzk);
-            dvdz = 0.5 * (dvdzL + dvdzR);
-            double dwdzL = (W[Lkp] - W[Lkm]) / (2.0 * dzk), dwdzR = (W[Rkp] - W[Rkm]) / (2.0 * dzk);
-            dwdz = 0.5 * (dwdzL + dwdzR);
-        }
-        double divU = dudx + dvdy + dwdz;
-        t0 = muF * (dudy + dvdx);
-        t1 = muF * (2.0 * dvdy - (2.0 / 3.0) * divU);
-        t2 = muF * (dwdy + dvdz);
-        double uF = 0.5 * (U[iL] + U[iR]), vF = 0.5 * (V[iL] + V[iR]), wF = 0.0;
-        if (dim >= 3) wF = 0.5 * (W[iL] + W[iR]);
-        work = t0 * uF + t1 * vF + t2 * wF;
-    } else {
-        double dzk = 0.5 * (F.dz[k - 1 + P.ngz] + F.dz[k + P.ngz]);
-        double dudz = (U[iR] - U[iL]) / dzk, dvdz = (V[iR] - V[iL]) / dzk, dwdz = (W[iR] - W[iL]) / dzk;
-        double dxi = F.dx[i + P.ngx];
-        size_t Lim = at(i - 1, j, k - 1), Lip = at(i + 1, j, k - 1), Rim = at(i - 1, j, k), Rip = at(i + 1, j, k);
-        double dudxL = (U[Lip] - U[Lim]) / (2.0 * dxi), dudxR = (U[Rip] - U[Rim]) / (2.0 * dxi);
-        double dudx = 0.5 * (dudxL + dudxR);
-        double dwdxL = (W[Lip] - W[Lim]) / (2.0 * dxi), dwdxR = (W[Rip] - W[Rim]) / (2.0 * dxi);
-        double dwdx = 0.5 * (dwdxL + dwdxR);
-        double dyj = F.dy[j + P.ngy];
-        size_t Ljm = at(i, j - 1, k - 1), Ljp = at(i, j + 1, k - 1), Rjm = at(i, j - 1, k), Rjp = at(i, j + 1, k);
-        double dvdyL = (V[Ljp] - V[Ljm]) / (2.0 * dyj), dvdyR = (V[Rjp] - V[Rjm]) / (2.0 * dyj);
-        double dvdy = 0.5 * (dvdyL + dvdyR);
-        double dwdyL = (W[Ljp] - W[Ljm]) / (2.0 * dyj), dwdyR = (W[Rjp] - W[Rjm]) / (2.0 * dyj);
-        double dwdy = 0.5 * (dwdyL + dwdyR);
-        double divU = dudx + dvdy + dwdz;
-        t0 = muF * (dudz + dwdx);
-        t1 = muF * (dvdz + dwdy);
-        t2 = muF * (2.0 * dwdz - (2.0 / 3.0) * divU);
-        double uF = 0.5 * (U[iL] + U[iR]), vF = 0.5 * (V[iL] + V[iR]), wF = 0.5 * (W[iL] + W[iR]);
-        work = t0 * uF + t1 * vF + t2 * wF;
-    }
+    double tau[3], work;
+    visc_stress<DIR>(dim, F.velU, F.velV, F.velW, iL, iR, (size_t)1, sy, sz, F.dx + i + P.ngx, F.dy + j + P.ngy,
+                     F.dz + k + P.ngz, muF, tau, work);
     double* const* out = F.flux[DIR] + FS_VISC;
-    out[0][t] = t0;
-    if (dim >= 2) out[1][t] = t1;
-    if (dim >= 3) out[2][t] = t2;
+    out[0][t] = tau[0];
+    if (dim >= 2) out[1][t] = tau[1];
+    if (dim >= 3) out[2][t] = tau[2];
     out[3][t] = work;
 }
 
@@ -763,14 +683,38 @@ __global__ void k_dt_init(Ctl* ctl, double maxDt) {
     ctl->dtBits = d2bits(maxDt);
 }
 
+// time += dt (src/RKTimeStepping.cpp:272-273); with an output interval, the
+// output test of runTimeLoop (275-277).  dtLog[slot]: the step's dt, or -1
+// for a skipped step.
+__device__ __forceinline__ void time_advance(Ctl* ctl, double* dtLog, int slot) {
+    if (ctl->skip) {
+        if (dtLog) dtLog[slot] = -1.0;
+        return;
+    }
+    ctl->time += ctl->dt;
+    ctl->stepsTaken += 1;
+    if (dtLog) dtLog[slot] = ctl->dt;
+    if (ctl->outInterval > 0.0 && ctl->time >= ctl->nextOutput - 1e-12 * ctl->outInterval) {
+        ctl->outputDue = 1;
+        ctl->nextOutput += ctl->outInterval;
+    }
+}
+
 // dt = min(maxDt, reduction); constDt; min with targetDt; semi-implicit
 // clamp (src/ExplicitSolver.cpp:72-90, src/SemiImplicitSolver.cpp:110-123).
 // useEnd 1: device-resident loop, targetDt = tEnd - time and steps past tEnd
 // are skipped.  useEnd 2: runTimeLoop (src/RKTimeStepping.cpp:259-266):
 // targetDt also capped at the next output time, and steps after the one
 // that reached an output are skipped until the host has handled it.
+// resetDt > 0: then start the accumulator of the next step at resetDt (the
+// last stage kernel folds that step's limits into it).  advance: first close
+// the previous step (time_advance).
 __global__ void k_dt_finalize(Ctl* ctl, double constDt, double targetDt, int clampSemi, double minDt, double maxDt,
-                              int useEnd) {
+                              int useEnd, double resetDt = 0.0, int advance = 0, double* dtLog = nullptr,
+                              int slot = 0) {
+    grid_dep_launch();
+    grid_dep_wait();
+    if (advance) time_advance(ctl, dtLog, slot);
     if (useEnd) {
         if (ctl->outputDue || !(ctl->time < ctl->tEnd)) {
             ctl->skip = 1;
@@ -784,24 +728,10 @@ __global__ void k_dt_finalize(Ctl* ctl, double constDt, double targetDt, int cla
     if (targetDt > 0) dt = smin(dt, targetDt);
     if (clampSemi) dt = (dt < minDt) ? minDt : (maxDt < dt) ? maxDt : dt;
     ctl->dt = dt;
+    if (resetDt > 0.0) ctl->dtBits = d2bits(resetDt);
 }
 
-// time += dt (src/RKTimeStepping.cpp:272-273); with an output interval, the
-// output test of runTimeLoop (275-277).  dtLog[slot]: the step's dt, or -1
-// for a skipped step.
-__global__ void k_time_advance(Ctl* ctl, double* dtLog = nullptr, int slot = 0) {
-    if (ctl->skip) {
-        if (dtLog) dtLog[slot] = -1.0;
-        return;
-    }
-    ctl->time += ctl->dt;
-    ctl->stepsTaken += 1;
-    if (dtLog) dtLog[slot] = ctl->dt;
-    if (ctl->outInterval > 0.0 && ctl->time >= ctl->nextOutput - 1e-12 * ctl->outInterval) {
-        ctl->outputDue = 1;
-        ctl->nextOutput += ctl->outInterval;
-    }
-}
+__global__ void k_time_advance(Ctl* ctl, double* dtLog = nullptr, int slot = 0) { time_advance(ctl, dtLog, slot); }
 
 // The host has written the output: steps run again.
 __global__ void k_loop_resume(Ctl* ctl) {
@@ -1800,30 +1730,6 @@ __global__ void __launch_bounds__(TY * TZ) k_igr_tile(Params P, Fields F, IgrPla
 // serial path of the wavefront.
 // ---------------------------------------------------------------------------
 
-// Correctly rounded a / b given y = RN(1 / b).  q0 = a y is within 1.5 ulp of
-// a / b; one residual correction q1 = RN(q0 + RN(a - b q0) y) is faithful
-// (within 1 ulp); Markstein's theorem (P. Markstein, "Computation of
-// elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
-// Dev. 34(1), 1990: for y = RN(1 / b) and a faithful q, r = a - b q is exact
-// and RN(q + r y) = RN(a / b)) makes the second correction the correctly
-// rounded quotient.  Valid when |y| lies in [2^-450, 2^450] and a is +0 or
-// |a| lies in [2^-450, 2^450] (quotient and residual then stay clear of
-// overflow and gradual underflow; a = +0 gives +0 or -0 as a / b does).
-// Callers check both with igr_fast_operand / igr_fast_recip and take the
-// plain division otherwise.
-__device__ __forceinline__ double div_markstein(double a, double b, double y) {
-    const double q0 = a * y;
-    const double q1 = fma(fma(-q0, b, a), y, q0);
-    return fma(fma(-q1, b, a), y, q1);
-}
-// |x| in [2^-450, 2^450] (biased exponent 573..1473)
-__device__ __forceinline__ bool igr_fast_recip(double x) {
-    return ((unsigned)__double2hiint(x) & 0x7ff00000u) - 0x23d00000u <= 0x38400000u;
-}
-// the same, or x = +0
-__device__ __forceinline__ bool igr_fast_operand(double x) {
-    return igr_fast_recip(x) || (((unsigned)__double2hiint(x) | (unsigned)__double2loint(x)) == 0u);
-}
 // igr_cell's update from staged values with plain divisions; kept out of
 // line so that the compiler does not if-convert it into the common path.
 __device__ __noinline__ double igr_cell_plain(double sxm, double sxp, double sym, double syp, double szm, double szp,
@@ -1892,7 +1798,7 @@ __global__ void __launch_bounds__(256) k_igr_records(Params P, Fields F, double*
     const double rxl = 1.0 / (0.5 * (rho_i + F.rho[c - 1]));
     if (n == ex) {
         o[0] = make_double2(rxl, 0.0);
-        if (!igr_fast_recip(rxl)) atomicOr(slowRecs, 1);
+        if (!rn_fast_recip(rxl)) atomicOr(slowRecs, 1);
         return;
     }
     const double diag = F.igrDiag[c];
@@ -1903,8 +1809,8 @@ __global__ void __launch_bounds__(256) k_igr_records(Params P, Fields F, double*
     o[kIgrTile] = make_double2(ryr, rzl);
     o[2 * kIgrTile] = make_double2(rzr, F.igrRhs[c]);
     o[3 * kIgrTile] = make_double2(diag, rd);
-    if (!(igr_fast_recip(rxl) && igr_fast_recip(ryl) && igr_fast_recip(ryr) && igr_fast_recip(rzl) &&
-          igr_fast_recip(rzr) && igr_fast_recip(rd)))
+    if (!(rn_fast_recip(rxl) && rn_fast_recip(ryl) && rn_fast_recip(ryr) && rn_fast_recip(rzl) &&
+          rn_fast_recip(rzr) && rn_fast_recip(rd)))
         atomicOr(slowRecs, 1);
 }
 
@@ -2034,14 +1940,14 @@ __global__ void __launch_bounds__(256, 1)
             const double rfly = 0.5 * (rho_i + sR[h - HXP]), rfry = 0.5 * (rho_i + sR[h + HXP]);
             const double rflz = 0.5 * (rho_i + sR[h - HXP * HY]), rfrz = 0.5 * (rho_i + sR[h + HXP * HY]);
             double v;
-            if (fastRecs && igr_fast_operand(sxm) && igr_fast_operand(sxp) && igr_fast_operand(sym) &&
-                igr_fast_operand(syp) && igr_fast_operand(szm) && igr_fast_operand(szp)) {
+            if (fastRecs && rn_fast_operand(sxm) && rn_fast_operand(sxp) && rn_fast_operand(sym) &&
+                rn_fast_operand(syp) && rn_fast_operand(szm) && rn_fast_operand(szp)) {
                 double off = 0.0;
                 off += sAx[a] * (div_markstein(sxm, rflx, c0.x) + div_markstein(sxp, rfrx, rxr));
                 off += ady * (div_markstein(sym, rfly, c0.y) + div_markstein(syp, rfry, c1.x));
                 off += adz * (div_markstein(szm, rflz, c1.y) + div_markstein(szp, rfrz, c2.x));
                 const double num = c2.y + off;
-                v = igr_fast_operand(num) ? div_markstein(num, c3.x, c3.y) : div_rn_plain(num, c3.x);
+                v = rn_fast_operand(num) ? div_markstein(num, c3.x, c3.y) : div_rn_plain(num, c3.x);
             } else {
                 v = igr_cell_plain(sxm, sxp, sym, syp, szm, szp, rflx, rfrx, rfly, rfry, rflz, rfrz, sAx[a], ady, adz,
                                    c2.y, c3.x);
@@ -2401,7 +2307,7 @@ __global__ void __launch_bounds__(256) k_gs_records(Params P, const double* __re
     o[2 * T] = make_double2(coef[4 * nc + c], coef[5 * nc + c]);
     o[3 * T] = make_double2(coef[6 * nc + c], denom);
     o[4 * T] = make_double2(rd, rhs[c]);
-    if (!igr_fast_recip(rd)) atomicOr(slowRecs, 1);
+    if (!rn_fast_recip(rd)) atomicOr(slowRecs, 1);
 }
 
 // One tile plane of Gauss-Seidel iteration `it` (a no-op once iteration
@@ -2478,7 +2384,7 @@ __global__ void __launch_bounds__(256, 1) k_gs_tile_rec(Params P, const double* 
             od += c1.x * sP[h - HXP] + c1.y * sP[h + HXP];
             od += c2.x * sP[h - HXP * HY] + c2.y * sP[h + HXP * HY];
             const double num = c4.y + c3.x * od;
-            const double pn = (fastRecs && igr_fast_operand(num)) ? div_markstein(num, c3.y, c4.x)
+            const double pn = (fastRecs && rn_fast_operand(num)) ? div_markstein(num, c3.y, c4.x)
                                                                   : div_rn_plain(num, c3.y);
             const double pOld = sP[h];
             sP[h] = pn;
@@ -2613,7 +2519,7 @@ __global__ void __launch_bounds__(256, 1) k_gs_tile_rec_ov(Params P, const doubl
             od += c1.x * sP[h - HXP] + c1.y * sP[h + HXP];
             od += c2.x * sP[h - HXP * HY] + c2.y * sP[h + HXP * HY];
             const double num = c4.y + c3.x * od;
-            const double pn = (fastRecs && igr_fast_operand(num)) ? div_markstein(num, c3.y, c4.x)
+            const double pn = (fastRecs && rn_fast_operand(num)) ? div_markstein(num, c3.y, c4.x)
                                                                   : div_rn_plain(num, c3.y);
             const double po = sP[h];
             sP[h] = pn;

@@ -89,3 +89,75 @@ def test_markstein_zero_numerator_sign():
     # would return +0 there
     assert not _operand_ok(-0.0)
     assert math.copysign(1.0, markstein(-0.0, 2.0, 0.5)) == 1.0
+
+
+# --- the quotients by the WENO5 weights (div_weight_rn, sifv_rn.cuh) --------------------------------------------
+# 2^(s + 1) A +- 1 for the significands A of 0.1 and 0.3 (0.6 has 0.3's), factored
+_FACTORS = {
+    (0.1, 52, 1): [7, 17, 23, 392028350279, 60489118407485863],
+    (0.1, 52, -1): [3, 44987759, 480899042868419303122811],
+    (0.1, 53, 1): [3, 3, 2007013, 1933980473, 3715820644449517],
+    (0.1, 53, -1): [5, 11, 2360134935697649053073123854969],
+    (0.3, 52, 1): [3, 7, 41, 41, 1319, 1269017, 823818512513339267],
+    (0.3, 52, -1): [19, 61, 919, 1979, 2657, 468523091, 18550836383],
+    (0.3, 53, 1): [325787358817, 298831625791270194593],
+    (0.3, 53, -1): [3, 3, 11, 499, 1970720554189753536002653879],
+}
+
+
+def _probable_prime(n: int) -> bool:
+    if n % 2 == 0:
+        return n == 2
+    d, r = n - 1, 0
+    while d % 2 == 0:
+        d, r = d // 2, r + 1
+    for a in (2, 3, 5, 7, 11, 13, 17, 19, 23, 29, 31, 37, 41):
+        if a % n == 0:
+            continue
+        x = pow(a, d, n)
+        if x in (1, n - 1):
+            continue
+        for _ in range(r - 1):
+            x = x * x % n
+            if x == n - 1:
+                break
+        else:
+            return False
+    return True
+
+
+@pytest.mark.parametrize("weight,s,d", sorted(_FACTORS))
+def test_no_divisor_defeats_the_weight_quotient(weight, s, d):
+    """A divisor B of 2^(s+1) A +- 1 above 0.98 2^53 would be a quotient one unit from a rounding boundary with a
+    reciprocal as far off as rcp_near allows; there is none."""
+    A = (_bits(weight) & ((1 << 52) - 1)) | (1 << 52)
+    assert _bits(0.6) & ((1 << 52) - 1) == _bits(0.3) & ((1 << 52) - 1)
+    primes = _FACTORS[(weight, s, d)]
+    n = 1
+    for p in primes:
+        assert _probable_prime(p)
+        n *= p
+    assert n == (A << (s + 1)) + d
+    divisors = {1}
+    for p in primes:
+        divisors |= {q * p for q in divisors}
+    assert not [b for b in divisors if 0.98 * 2 ** 53 < b < 2 ** 53 and 2 ** 53 < n // b < 2 ** 54]
+
+
+@pytest.mark.parametrize("seed", [0, 1])
+def test_weight_quotient_matches_ieee_division(seed):
+    """The quotient with a reciprocal up to half an ulp plus 2^-6 ulp off (both neighbours of 1 / b where b's
+    reciprocal lies near their midpoint) against the exact one."""
+    from fractions import Fraction
+    rng = np.random.default_rng(seed)
+    for k in range(20000):
+        mb = int(rng.integers(0, 1 << 52))
+        if k % 3 == 1:
+            mb = (1 << 52) - 1 - (mb & 0xFFF)
+        b = struct.unpack("<d", struct.pack("<q", ((1023 + int(rng.integers(-60, 60))) << 52) | mb))[0]
+        y = 1.0 / b
+        for yy in (y, math.nextafter(y, 0.0), math.nextafter(y, math.inf)):
+            if abs(Fraction(yy) - 1 / Fraction(b)) > (Fraction(1, 2) + Fraction(1, 64)) * Fraction(math.ulp(y)):
+                continue
+            for a in (0.1, 0.6, 0.3):
+                assert markstein(a, b, yy) == a / b
