@@ -1,4 +1,6 @@
 // sifv_adjoint.cu -- launchers of the discrete adjoint and tangent kernels.
+#include <algorithm>
+
 #include "sifv_adjoint.cuh"
 
 namespace sifv {
@@ -12,18 +14,31 @@ long long nfaces(const Params& P, int d) {
 }
 
 template <int DIM, typename S>
-void adj_faces(const AdjArgs& A, cudaStream_t s) {
-    k_adj_face<0, DIM, S><<<nblocks(nfaces(A.P, 0), 128), 128, 0, s>>>(A);
-    if (DIM >= 2) k_adj_face<(DIM >= 2 ? 1 : 0), DIM, S><<<nblocks(nfaces(A.P, 1), 128), 128, 0, s>>>(A);
-    if (DIM >= 3) k_adj_face<(DIM >= 3 ? 2 : 0), DIM, S><<<nblocks(nfaces(A.P, 2), 128), 128, 0, s>>>(A);
+int adj_dirs(const AdjArgs& A, cudaStream_t s) {
+    constexpr size_t smem = adj_dir_smem<DIM, S>();
+    if (cudaFuncSetAttribute(k_adj_dir<DIM, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        return -1;
+    const Params& P = A.P;
+    const long long n[3] = {P.nx, P.ny, P.nz};
+    long long tiles = 0, lines = 0;
+    for (int d = 0; d < DIM; ++d) {
+        tiles = std::max(tiles, (n[d] + 6 + kAdjOut - 1) / kAdjOut);
+        lines = std::max(lines, n[0] * n[1] * n[2] / n[d]);
+    }
+    const long long groups = (lines + kAdjLines - 1) / kAdjLines;
+    if (tiles * groups > 0x7fffffffLL) return -1;
+    AdjArgs B = A;
+    B.adjTiles = (unsigned)tiles;
+    k_adj_dir<DIM, S><<<dim3((unsigned)(tiles * groups), DIM), kAdjLines * kAdjLen, smem, s>>>(B);
+    return 0;
 }
 
 template <int DIM>
-void adj_stage(const AdjArgs& A, cudaStream_t s) {
-    if (A.fp32) adj_faces<DIM, float>(A, s);
-    else adj_faces<DIM, double>(A, s);
+int adj_stage(const AdjArgs& A, cudaStream_t s) {
+    if ((A.fp32 ? adj_dirs<DIM, float>(A, s) : adj_dirs<DIM, double>(A, s)) != 0) return -1;
     const long long n = (long long)A.P.nx * A.P.ny * A.P.nz;
     k_adj_cell<DIM><<<nblocks(n, 128), 128, 0, s>>>(A);
+    return 0;
 }
 
 template <int DIM>
@@ -45,11 +60,8 @@ __global__ void k_zero_ghosts(Params P, double* f) {
 }  // namespace
 
 int adjoint_stage(const AdjArgs& A, cudaStream_t s) {
-    switch (A.P.dim) {
-        case 1: adj_stage<1>(A, s); break;
-        case 2: adj_stage<2>(A, s); break;
-        default: adj_stage<3>(A, s); break;
-    }
+    const int st = (A.P.dim == 1) ? adj_stage<1>(A, s) : (A.P.dim == 2) ? adj_stage<2>(A, s) : adj_stage<3>(A, s);
+    if (st != 0) return st;
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

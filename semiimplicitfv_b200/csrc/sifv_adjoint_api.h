@@ -13,10 +13,11 @@ struct AdjArgs {
     Fields F;            // stage input: cons (and prims incl. ghosts once filled)
     double* lam[5];      // dJ/dU' in, dJ/dU out (rho, momenta, rhoE; interior cells)
     double* acc0[5];     // dJ/dU0 accumulated through the RK combination
-    double* share[3];    // per direction: 10 * (dim + 2) doubles per face
+    double* gdir[3][5];  // dJ/dW per direction (all cells; ghost positions within three layers)
     double dt, a1, a2, a3;   // dt and c1/c4, c2/c4, c3/c4 of the stage
     const double* dtDev;     // non-null: dt is read from device memory (the step's CFL dt)
     int stage0;          // stage 0 of a step: lam += acc0, acc0 = 0
+    unsigned adjTiles;   // blocks along a grid line of the reverse kernel (set by the launcher)
     int fp32;            // local Jacobians of the reverse sweep in FP32
     double* tan[5];      // tangent dU (interior cells)
     double* tan0[5];     // tangent of the step-start state
@@ -24,7 +25,7 @@ struct AdjArgs {
     double* tanF[3][5];  // tangent face fluxes per direction
 };
 
-// Reverse of one RK stage (prims of the stage input must be filled).
+// Reverse of one RK stage (F: the conservative stage input).
 int adjoint_stage(const AdjArgs& A, cudaStream_t s);
 // Tangent of one stage before the forward update (prim + face tangents) and
 // after it (the RK combination; save = stage 0 of a multi-stage step).

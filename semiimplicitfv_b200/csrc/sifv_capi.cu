@@ -79,7 +79,7 @@ struct sifv_ctx {
     sifv_comm_t comm{};                       // halo exchange / dt reduction of a decomposed run
     int adjEvery = 0;
     std::vector<double> adjDts;               // time-step sequence of the recorded forward run
-    std::vector<double*> adjCkpt;             // (dim + 2) arrays per checkpoint, then the final state
+    std::vector<double*> adjCkpt;             // dim + 2 fields per checkpoint, then the final state
     double* adjStage = nullptr;               // stage inputs of one segment
     size_t adjStageCap = 0;
     bool adjReady = false;
@@ -111,7 +111,8 @@ struct sifv_ctx {
     int advSlot = 0;
     double* lam[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     double* acc0[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
-    double* share[3] = {nullptr, nullptr, nullptr};
+    double* gdir[3][5] = {};                  // dJ/dW per direction of the reverse sweep
+    std::vector<double*> adjPool;             // checkpoints not in use (kept between forward runs)
     double* tan[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     double* tan0[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     double* tanW[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -2057,6 +2058,7 @@ int sifv_destroy(sifv_ctx_t* c) {
     if (c->ev1) cudaEventDestroy(c->ev1);
     if (c->ownStream) cudaStreamDestroy(c->ownStream);
     for (double* p : c->adjCkpt) cudaFree(p);
+    for (double* p : c->adjPool) cudaFree(p);
     if (c->adjStage) cudaFree(c->adjStage);
     if (c->loopLog) cudaFree(c->loopLog);
     for (void* p : c->ibAllocs) cudaFree(p);
@@ -2449,7 +2451,8 @@ int ensure_adj_arrays(sifv_ctx* c, bool tangent) {
             c->lam[q] = dalloc(c, c->ncells, st);
             c->acc0[q] = dalloc(c, c->ncells, st);
         }
-        for (int d = 0; d < dim; ++d) c->share[d] = dalloc(c, face_count(c->P, d) * 10 * nv, st);
+        for (int d = 0; d < dim; ++d)
+            for (int q = 0; q < nv; ++q) c->gdir[d][q] = dalloc(c, c->ncells, st);
     }
     if (tangent && !c->tan[0]) {
         for (int q = 0; q < nv; ++q) {
@@ -2475,8 +2478,10 @@ AdjArgs adj_args(sifv_ctx* c) {
         A.tanW[q] = c->tanW[q];
     }
     for (int d = 0; d < 3; ++d) {
-        A.share[d] = c->share[d];
-        for (int q = 0; q < 5; ++q) A.tanF[d][q] = c->tanF[d][q];
+        for (int q = 0; q < 5; ++q) {
+            A.gdir[d][q] = c->gdir[d][q];
+            A.tanF[d][q] = c->tanF[d][q];
+        }
     }
     A.fp32 = c->adjFp32;
     return A;
@@ -2490,8 +2495,11 @@ void set_stage_coef(AdjArgs& A, int order, int s) {
     A.a3 = K.c3 / K.c4;
 }
 
+// Checkpoint arrays go back to the context's pool: the next forward run of a
+// program that differentiates repeatedly takes them from there instead of
+// allocating and freeing device memory (which waits for the device) anew.
 void free_checkpoints(sifv_ctx* c) {
-    for (double* p : c->adjCkpt) cudaFree(p);
+    c->adjPool.insert(c->adjPool.end(), c->adjCkpt.begin(), c->adjCkpt.end());
     c->adjCkpt.clear();
     c->adjDts.clear();
     c->adjReady = false;
@@ -2499,11 +2507,16 @@ void free_checkpoints(sifv_ctx* c) {
 
 // copy of the conservative state appended to the checkpoint list
 int push_checkpoint(sifv_ctx* c) {
-    for (int q = 0; q < nv_of(c); ++q) {
+    if (c->adjPool.empty()) {
         void* p = nullptr;
-        if (cudaMalloc(&p, c->ncells * sizeof(double)) != cudaSuccess)
+        if (cudaMalloc(&p, (size_t)nv_of(c) * c->ncells * sizeof(double)) != cudaSuccess)
             return fail(c, SIFV_ERR_CUDA, "cudaMalloc for an adjoint checkpoint failed");
-        c->adjCkpt.push_back(static_cast<double*>(p));
+        c->adjPool.push_back(static_cast<double*>(p));
+    }
+    c->adjCkpt.push_back(c->adjPool.back());
+    c->adjPool.pop_back();
+    for (int q = 0; q < nv_of(c); ++q) {
+        double* p = c->adjCkpt.back() + (size_t)q * c->ncells;
         CUDA_TRY(c, cudaMemcpyAsync(p, cons_field(c, q), c->ncells * sizeof(double), cudaMemcpyDeviceToDevice,
                                     c->stream));
     }
@@ -2513,7 +2526,7 @@ int push_checkpoint(sifv_ctx* c) {
 int load_checkpoint(sifv_ctx* c, size_t idx) {
     const int nv = nv_of(c);
     for (int q = 0; q < nv; ++q)
-        CUDA_TRY(c, cudaMemcpyAsync(cons_field(c, q), c->adjCkpt[idx * nv + q], c->ncells * sizeof(double),
+        CUDA_TRY(c, cudaMemcpyAsync(cons_field(c, q), c->adjCkpt[idx] + (size_t)q * c->ncells, c->ncells * sizeof(double),
                                     cudaMemcpyDeviceToDevice, c->stream));
     return SIFV_OK;
 }
@@ -2528,35 +2541,60 @@ struct HookGuard {
 
 // Forward steps from the current state, either with a given time-step
 // sequence or with the CFL dt and targetDt = tEnd - t; optionally records
-// the sequence and a checkpoint every `every` steps.
+// the sequence and a checkpoint every `every` steps.  The steps between two
+// checkpoints (64 at most) run device-resident, the device logging their dts;
+// the host reads the log once per batch.
 int run_forward(sifv_ctx* c, int step0, double time0, double tEnd, int maxSteps, const double* sched, int nSched,
                 int every, bool record, double& timeOut, int& stepsOut) {
     double t = time0;
     int q = 0;
     c->dtReady = false;   // the state may have changed since the last call
+    double lastDt = 0.0;
+    const int batchMax = record ? std::min(every, 64) : 64;
+    int ls = loop_log(c, batchMax);
+    if (ls != SIFV_OK) return ls;
+    std::vector<double> log(batchMax);
+    Ctl h{};
+    h.time = time0;
+    h.tEnd = sched ? INFINITY : tEnd;
+    CUDA_TRY(c, cudaMemcpyAsync(c->ctl, &h, offsetof(Ctl, res), cudaMemcpyHostToDevice, c->stream));
     for (;;) {
-        if (sched) {
-            if (q >= nSched) break;
-        } else if (!(t < tEnd) || (maxSteps > 0 && q >= maxSteps)) {
-            break;
-        }
+        int left = sched ? nSched - q : (maxSteps > 0) ? maxSteps - q : batchMax;
+        if (left <= 0 || (!sched && !(t < tEnd))) break;
         if (record && q % every == 0) {
             int st = push_checkpoint(c);
             if (st != SIFV_OK) return st;
         }
-        c->forcedDt = sched ? sched[q] : -1.0;
-        CUDA_TRY(c, cudaMemsetAsync(&c->ctl->skip, 0, sizeof(int), c->stream));
-        int status = SIFV_OK;
-        int st = enqueue_step(c, step0 + q, t, sched ? -1.0 : tEnd - t, false, status);
-        c->forcedDt = -1.0;
-        if (st != SIFV_OK) return st;
-        CUDA_TRY(c, cudaMemcpyAsync(c->ctlHost, c->ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, c->stream));
+        int B = std::min(left, batchMax);
+        if (record) B = std::min(B, every - q % every);
+        // steps past tEnd would be queued for nothing: one step first, then as many as its dt suggests
+        if (!sched) B = (lastDt > 0.0) ? (int)std::min<double>(B, std::floor((tEnd - t) / lastDt) + 1.0) : 1;
+        for (int b = 0; b < B; ++b) {
+            c->forcedDt = sched ? sched[q + b] : -1.0;
+            int status = SIFV_OK;
+            int st = enqueue_step(c, step0 + q + b, t, -1.0, sched ? 0 : 1, status);
+            c->forcedDt = -1.0;
+            if (st != SIFV_OK) {
+                c->advPending = false;
+                return st;
+            }
+            c->advPending = true;
+            c->advLog = c->loopLog;
+            c->advSlot = b;
+        }
+        flush_advance(c);
+        CUDA_TRY(c, cudaMemcpyAsync(log.data(), c->loopLog, sizeof(double) * B, cudaMemcpyDeviceToHost, c->stream));
         CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-        const double dt = c->ctlHost->dt;
-        if (!(dt > 0.0)) return fail(c, SIFV_ERR_NAN, "time step not positive (state blew up)");
-        if (record) c->adjDts.push_back(dt);
-        t += dt;
-        ++q;
+        for (int b = 0; b < B; ++b) {
+            // a step past tEnd logs -1; any other dt that is not positive is a blown-up state
+            if (!sched && !(t < tEnd)) break;
+            const double dt = log[b];
+            if (!(dt > 0.0)) return fail(c, SIFV_ERR_NAN, "time step not positive (state blew up)");
+            if (record) c->adjDts.push_back(dt);
+            t += dt;
+            lastDt = dt;
+            ++q;
+        }
     }
     timeOut = t;
     stepsOut = q;
@@ -2611,6 +2649,8 @@ int sifv_adjoint_forward(sifv_ctx_t* c, int step0, double time0, double tEnd, in
     }
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     c->adjReady = true;
+    for (double* p : c->adjPool) cudaFree(p);   // no more is kept than this run used
+    c->adjPool.clear();
     if (timeOut) *timeOut = t;
     if (stepsOut) *stepsOut = n;
     return SIFV_OK;
@@ -2658,7 +2698,7 @@ int sifv_adjoint_backward(sifv_ctx_t* c, double* deviceMs) {
     const int nv = nv_of(c), RK = c->cfg.RKOrder, K = c->adjEvery, dim = c->cfg.dim;
     const int nSteps = (int)c->adjDts.size();
     const size_t nc = c->ncells;
-    const size_t need = (size_t)K * RK * nv * nc;
+    const size_t need = (size_t)std::min(K, std::max(nSteps, 1)) * RK * nv * nc;
     if (c->adjStageCap < need) {
         if (c->adjStage) cudaFree(c->adjStage);
         c->adjStage = nullptr;
@@ -2675,29 +2715,55 @@ int sifv_adjoint_backward(sifv_ctx_t* c, double* deviceMs) {
     const int nSeg = (nSteps + K - 1) / K;
     for (int seg = nSeg - 1; seg >= 0; --seg) {
         const int q0 = seg * K, q1 = std::min(q0 + K, nSteps);
-        st = load_checkpoint(c, (size_t)seg);
-        if (st != SIFV_OK) return st;
         // recompute the segment, keeping every stage input
-        int qLocal = 0;
-        c->stageHook = [&](int s, int phase) -> int {
-            if (phase != 0) return 0;
-            double* dst = c->adjStage + (size_t)(qLocal * RK + s) * nv * nc;
+        if (fused_stage(c)) {
+            // the stage kernel writes each stage's output where the next stage's input is kept
+            auto kept = [&](int slot) {
+                StageState S{};
+                double* base = c->adjStage + (size_t)slot * nv * nc;
+                S.rho = base;
+                for (int d = 0; d < dim; ++d) S.mom[d] = base + (size_t)(1 + d) * nc;
+                S.rhoE = base + (size_t)(dim + 1) * nc;
+                return S;
+            };
             for (int v = 0; v < nv; ++v)
-                if (cudaMemcpyAsync(dst + v * nc, cons_field(c, v), nc * sizeof(double), cudaMemcpyDeviceToDevice,
-                                    c->stream) != cudaSuccess)
-                    return -1;
-            return 0;
-        };
-        for (int q = q0; q < q1; ++q) {
-            qLocal = q - q0;
-            c->forcedDt = c->adjDts[q];
-            CUDA_TRY(c, cudaMemsetAsync(&c->ctl->skip, 0, sizeof(int), c->stream));
-            int status = SIFV_OK;
-            st = enqueue_step(c, q, 0.0, -1.0, false, status);
+                CUDA_TRY(c, cudaMemcpyAsync(c->adjStage + v * nc, c->adjCkpt[(size_t)seg] + (size_t)v * nc, nc * sizeof(double),
+                                            cudaMemcpyDeviceToDevice, c->stream));
+            for (int q = q0; q < q1; ++q)
+                for (int s = 0; s < RK; ++s) {
+                    const int slot = (q - q0) * RK + s;
+                    if (slot + 1 == (q1 - q0) * RK) break;   // the segment's end is the next checkpoint
+                    StageArgs A = stage_args(c, s);
+                    A.dtFixed = c->adjDts[q];
+                    A.in = kept(slot);
+                    A.u0 = kept((q - q0) * RK);
+                    A.out = kept(slot + 1);
+                    if (stage_launch(A, c->stream) != 0) return fail(c, SIFV_ERR_CUDA, "stage launch failed");
+                }
+        } else {
+            st = load_checkpoint(c, (size_t)seg);
             if (st != SIFV_OK) return st;
+            int qLocal = 0;
+            c->stageHook = [&](int s, int phase) -> int {
+                if (phase != 0) return 0;
+                double* dst = c->adjStage + (size_t)(qLocal * RK + s) * nv * nc;
+                for (int v = 0; v < nv; ++v)
+                    if (cudaMemcpyAsync(dst + v * nc, cons_field(c, v), nc * sizeof(double), cudaMemcpyDeviceToDevice,
+                                        c->stream) != cudaSuccess)
+                        return -1;
+                return 0;
+            };
+            for (int q = q0; q < q1; ++q) {
+                qLocal = q - q0;
+                c->forcedDt = c->adjDts[q];
+                CUDA_TRY(c, cudaMemsetAsync(&c->ctl->skip, 0, sizeof(int), c->stream));
+                int status = SIFV_OK;
+                st = enqueue_step(c, q, 0.0, -1.0, false, status);
+                if (st != SIFV_OK) return st;
+            }
+            c->stageHook = nullptr;
+            c->forcedDt = -1.0;
         }
-        c->stageHook = nullptr;
-        c->forcedDt = -1.0;
         // reverse through the segment
         for (int q = q1 - 1; q >= q0; --q) {
             for (int s = RK - 1; s >= 0; --s) {
@@ -2708,7 +2774,6 @@ int sifv_adjoint_backward(sifv_ctx_t* c, double* deviceMs) {
                 if (dim >= 2) Fs.rhoV = src + 2 * nc;
                 if (dim >= 3) Fs.rhoW = src + 3 * nc;
                 Fs.rhoE = src + (size_t)(dim + 1) * nc;
-                k_prim_bc<0><<<blocks((long long)nc, kCellThreads), kCellThreads, 0, c->stream>>>(c->P, Fs, nullptr, 0);
                 AdjArgs A = adj_args(c);
                 A.F = Fs;
                 set_stage_coef(A, RK, s);
