@@ -28,7 +28,7 @@ struct sifv_ensemble {
     std::vector<void*> allocs;
     std::vector<long long> off;
     long long ncells = 0;
-    int blockSize = 256;
+    int blockSize = 512;
     std::string err;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 };
@@ -71,11 +71,7 @@ double* efield(sifv_ensemble* e, int f) {
 
 template <typename T, int NPH>
 int launch_t(const EnsArgs& A, int blockSize, cudaStream_t s) {
-    const size_t bytes = ens_smem_bytes<T, NPH>(blockSize);
-    if (cudaFuncSetAttribute(k_ensemble<T, NPH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) !=
-        cudaSuccess)
-        return -1;
-    k_ensemble<T, NPH><<<A.nInst, blockSize, bytes, s>>>(A);
+    k_ensemble<T, NPH><<<A.nInst, blockSize, 0, s>>>(A);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -87,23 +83,10 @@ int launch(sifv_ensemble* e, int blockSize) {
     return launch_t<double, 8>(e->A, blockSize, e->stream);
 }
 
-// dynamic shared memory of one block, and the largest usable block size
-size_t smem_bytes(const sifv_ensemble* e, int blockSize) {
-    const bool f = e->cfg.precision == SIFV_PREC_MIXED;
-    switch (e->nphT) {
-        case 0: return f ? ens_smem_bytes<float, 0>(blockSize) : ens_smem_bytes<double, 0>(blockSize);
-        case 2: return f ? ens_smem_bytes<float, 2>(blockSize) : ens_smem_bytes<double, 2>(blockSize);
-        default: return f ? ens_smem_bytes<float, 8>(blockSize) : ens_smem_bytes<double, 8>(blockSize);
-    }
-}
-
+// the largest usable block size
 int max_block(const sifv_ensemble* e) {
-    int dev = 0, optin = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    int m = (e->cfg.precision == SIFV_PREC_MIXED) ? 1024 : 512;
-    while (m > 32 && smem_bytes(e, m) + 512 > (size_t)optin) m -= 32;
-    return m;
+    if (e->cfg.precision != SIFV_PREC_MIXED) return EnsMaxThreads<double, 0>::value;
+    return (e->nphT > 2) ? EnsMaxThreads<float, 8>::value : EnsMaxThreads<float, 2>::value;
 }
 
 // all packed state arrays (for the autotuner's save / restore)
@@ -209,6 +192,22 @@ int sifv_ensemble_create(const sifv_config_t* cfg, int nInst, const int* nCells,
         if (cudaStreamSynchronize(e->stream) != cudaSuccess) st = efail(e, SIFV_ERR_CUDA, "upload failed");
     }
     A.order = ord; A.n = nn; A.off = offd;
+    if (cfg->precision == SIFV_PREC_MIXED && e->nphT <= 2) {
+        // Default block size of a mixed run: 512 threads (two instances per SM) unless the longest instance
+        // (cost n^2, steps going with n) would outlast three times an even split of all of them over the GPU's
+        // warps; then 1024, which halves its chain.  40 steps of 400 tubes of 256 - 4096 cells (ratio 4.1):
+        // 6.18 ms at 512, 4.23 at 1024; 400 of 200 - 800 (2.2): 1.50, 1.74; 2048 of 256 - 4096 (0.8), 10 steps:
+        // 5.14, 5.33.  FP64 runs at most 512 and is fastest there (14.2 ms, 25.5 at 256).
+        int sms = 148;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+        double sum = 0.0, top = 0.0;
+        for (int k = 0; k < nInst; ++k) {
+            const double w = (double)nCells[k] * nCells[k];
+            sum += w;
+            top = std::max(top, w);
+        }
+        if (top / 16.0 > 3.0 * sum / (32.0 * sms)) e->blockSize = 1024;
+    }
     Params& P = A.P;
     P.dim = 1; P.ny = P.nz = 1; P.ngx = ng; P.ngy = P.ngz = 0; P.nyT = P.nzT = 1;
     P.bc[0] = bc[0]; P.bc[1] = bc[1];
@@ -223,7 +222,13 @@ int sifv_ensemble_create(const sifv_config_t* cfg, int nInst, const int* nCells,
     P.wenoEps = cfg->wenoEps;
     P.gamma = cfg->gamma;
     P.pInf = P.eosStiffened ? cfg->pInf : 0.0;
-    for (int p = 0; p < SIFV_MAX_PHASES; ++p) { P.phaseGamma[p] = cfg->phaseGamma[p]; P.phasePInf[p] = cfg->phasePInf[p]; }
+    for (int p = 0; p < SIFV_MAX_PHASES; ++p) {
+        P.phaseGamma[p] = cfg->phaseGamma[p];
+        P.phasePInf[p] = cfg->phasePInf[p];
+        const double gm1 = cfg->phaseGamma[p] - 1.0;
+        e->A.invGm1[p] = (p < cfg->nPhases) ? 1.0 / gm1 : 0.0;
+        e->A.gPiGm1[p] = (p < cfg->nPhases) ? cfg->phaseGamma[p] * cfg->phasePInf[p] / gm1 : 0.0;
+    }
     P.alphaMin = cfg->alphaMin;
     A.cfl = cfg->cfl; A.maxDt = cfg->maxDt; A.constDt = cfg->constDt;
     if (st != SIFV_OK) {
@@ -303,7 +308,7 @@ int sifv_ensemble_run(sifv_ensemble_t* e, double tEnd, int maxSteps, int blockSi
 }
 
 // Pick the block size (128 / 256 / 512 threads per instance, and 1024 with
-// FP32 bulk, as shared memory allows) with the shortest time for a probe in
+// FP32 bulk) with the shortest time for a probe in
 // which every instance takes steps in proportion to its cell count (as in a
 // run to a common end time at a fixed CFL), the largest probeSteps steps;
 // the state is restored afterwards.
@@ -327,7 +332,7 @@ int sifv_ensemble_autotune(sifv_ensemble_t* e, int probeSteps, int* blockSizeOut
     cudaMemcpyAsync(t0.data(), e->A.time, e->nInst * sizeof(double), cudaMemcpyDeviceToHost, e->stream);
     cudaMemcpyAsync(s0.data(), e->A.steps, e->nInst * sizeof(int), cudaMemcpyDeviceToHost, e->stream);
     cudaStreamSynchronize(e->stream);
-    int best = 256;
+    int best = e->blockSize;
     float bestMs = 1e30f;
     const int cands[4] = {128, 256, 512, 1024};
     const int maxBs = max_block(e);

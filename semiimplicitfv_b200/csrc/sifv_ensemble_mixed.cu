@@ -12,11 +12,7 @@ namespace sifv {
 namespace {
 template <int NPH>
 int launch_f(const EnsArgs& A, int blockSize, cudaStream_t s) {
-    const size_t bytes = ens_smem_bytes<float, NPH>(blockSize);
-    if (cudaFuncSetAttribute(k_ensemble<float, NPH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) !=
-        cudaSuccess)
-        return -1;
-    k_ensemble<float, NPH><<<A.nInst, blockSize, bytes, s>>>(A);
+    k_ensemble<float, NPH><<<A.nInst, blockSize, 0, s>>>(A);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 }  // namespace
