@@ -65,51 +65,50 @@ __device__ __forceinline__ float frsqrt_pos(float x) {
 // Both WENO5 face values of the cell whose 5-cell stencil is v0..v4
 // (v2 = the cell): L = value at its right face from the left,
 // R = value at its left face from the right.
+//
+// In terms of the four differences d: the indicators times four are
+// 13/3 t^2 + s^2 with t, s one operation each, and since the weights sum to
+// one the candidates enter as their offsets from v2 (times six; the 1/6 goes
+// into the normalisation).  The linear weights count as 1 : 6 : 3.
+// 56 operations and two reciprocals where the form in cell values took 77
+// (fused 2D stage at 4096^2: 3.84 -> 3.26 ms per step).
 __device__ __forceinline__ void weno5_pair(double v0, double v1, double v2, double v3, double v4, double eps,
                                            double& L, double& R) {
-    double t0 = v0 - 2.0 * v1 + v2, s0 = v0 - 4.0 * v1 + 3.0 * v2;
-    double t1 = v1 - 2.0 * v2 + v3, s1 = v1 - v3;
-    double t2 = v2 - 2.0 * v3 + v4, s2 = 3.0 * v2 - 4.0 * v3 + v4;
-    double q0 = eps + ((13.0 / 12.0) * t0 * t0 + 0.25 * s0 * s0);
-    double q1 = eps + ((13.0 / 12.0) * t1 * t1 + 0.25 * s1 * s1);
-    double q2 = eps + ((13.0 / 12.0) * t2 * t2 + 0.25 * s2 * s2);
+    const double d0 = v1 - v0, d1 = v2 - v1, d2 = v3 - v2, d3 = v4 - v3;
+    const double t0 = d1 - d0, t1 = d2 - d1, t2 = d3 - d2;
+    const double s0 = fma(3.0, d1, -d0), s1 = d1 + d2, s2 = fma(-3.0, d2, d3);
+    const double e = 4.0 * eps;
+    double q0 = fma(s0, s0, fma((13.0 / 3.0) * t0, t0, e));
+    double q1 = fma(s1, s1, fma((13.0 / 3.0) * t1, t1, e));
+    double q2 = fma(s2, s2, fma((13.0 / 3.0) * t2, t2, e));
     q0 *= q0; q1 *= q1; q2 *= q2;
     // a_k = d_k / q_k; multiplying through by q0 q1 q2 leaves one division per side
-    double m01 = q0 * q1, m02 = q0 * q2, m12 = q1 * q2;
-    // candidate polynomials times 6; the 1/6 goes into the normalisation
-    double pL0 = 2.0 * v0 - 7.0 * v1 + 11.0 * v2;
-    double pL1 = -v1 + 5.0 * v2 + 2.0 * v3;
-    double pL2 = 2.0 * v2 + 5.0 * v3 - v4;
-    double pR0 = 2.0 * v4 - 7.0 * v3 + 11.0 * v2;
-    double pR1 = -v3 + 5.0 * v2 + 2.0 * v1;
-    double pR2 = 2.0 * v2 + 5.0 * v1 - v0;
-    double wL0 = 0.1 * m12, wL1 = 0.6 * m02, wL2 = 0.3 * m01;   // L: d = (.1,.6,.3) on (b0,b1,b2)
-    double wR0 = 0.1 * m01, wR1 = 0.6 * m02, wR2 = 0.3 * m12;   // R: d = (.1,.6,.3) on (b2,b1,b0)
-    L = (wL0 * pL0 + wL1 * pL1 + wL2 * pL2) * frcp(6.0 * (wL0 + wL1 + wL2));
-    R = (wR0 * pR0 + wR1 * pR1 + wR2 * pR2) * frcp(6.0 * (wR0 + wR1 + wR2));
+    const double m01 = q0 * q1, m12 = q1 * q2, c1 = 6.0 * (q0 * q2);
+    const double l2 = 3.0 * m01, r0 = 3.0 * m12;   // L: (1, 6, 3) on (q0, q1, q2); R: (3, 6, 1)
+    const double nL = fma(l2, fma(4.0, d2, -d3), fma(c1, fma(2.0, d2, d1), m12 * fma(5.0, d1, -2.0 * d0)));
+    const double nR = fma(r0, fma(4.0, d1, -d0), fma(c1, fma(2.0, d1, d2), m01 * fma(5.0, d2, -2.0 * d3)));
+    L = fma(nL, frcp(6.0 * ((m12 + c1) + l2)), v2);
+    R = fma(-nR, frcp(6.0 * ((m01 + c1) + r0)), v2);
 }
 
 // FP32 version: the product form would overflow single precision for
-// large-valued fields (q ~ (dp^2)^2), so the weights use reciprocals.
+// large-valued fields (q ~ (dp^2)^2), so the weights use reciprocals (of
+// q^2 / 16, which overflows no earlier than the indicators' own squares).
 __device__ __forceinline__ void weno5_pair(float v0, float v1, float v2, float v3, float v4, float eps, float& L,
                                            float& R) {
-    float t0 = v0 - 2.0f * v1 + v2, s0 = v0 - 4.0f * v1 + 3.0f * v2;
-    float t1 = v1 - 2.0f * v2 + v3, s1 = v1 - v3;
-    float t2 = v2 - 2.0f * v3 + v4, s2 = 3.0f * v2 - 4.0f * v3 + v4;
-    float q0 = eps + ((13.0f / 12.0f) * t0 * t0 + 0.25f * s0 * s0);
-    float q1 = eps + ((13.0f / 12.0f) * t1 * t1 + 0.25f * s1 * s1);
-    float q2 = eps + ((13.0f / 12.0f) * t2 * t2 + 0.25f * s2 * s2);
-    float r0 = frcp(q0 * q0), r1 = frcp(q1 * q1), r2 = frcp(q2 * q2);
-    float pL0 = (2.0f * v0 - 7.0f * v1 + 11.0f * v2) * (1.0f / 6.0f);
-    float pL1 = (-v1 + 5.0f * v2 + 2.0f * v3) * (1.0f / 6.0f);
-    float pL2 = (2.0f * v2 + 5.0f * v3 - v4) * (1.0f / 6.0f);
-    float pR0 = (2.0f * v4 - 7.0f * v3 + 11.0f * v2) * (1.0f / 6.0f);
-    float pR1 = (-v3 + 5.0f * v2 + 2.0f * v1) * (1.0f / 6.0f);
-    float pR2 = (2.0f * v2 + 5.0f * v1 - v0) * (1.0f / 6.0f);
-    float aL0 = 0.1f * r0, aL1 = 0.6f * r1, aL2 = 0.3f * r2;
-    float aR0 = 0.1f * r2, aR1 = 0.6f * r1, aR2 = 0.3f * r0;
-    L = (aL0 * pL0 + aL1 * pL1 + aL2 * pL2) * frcp(aL0 + aL1 + aL2);
-    R = (aR0 * pR0 + aR1 * pR1 + aR2 * pR2) * frcp(aR0 + aR1 + aR2);
+    const float d0 = v1 - v0, d1 = v2 - v1, d2 = v3 - v2, d3 = v4 - v3;
+    const float t0 = d1 - d0, t1 = d2 - d1, t2 = d3 - d2;
+    const float s0 = fmaf(3.0f, d1, -d0), s1 = d1 + d2, s2 = fmaf(-3.0f, d2, d3);
+    const float e = 4.0f * eps;
+    const float q0 = fmaf(s0, s0, fmaf((13.0f / 3.0f) * t0, t0, e));
+    const float q1 = fmaf(s1, s1, fmaf((13.0f / 3.0f) * t1, t1, e));
+    const float q2 = fmaf(s2, s2, fmaf((13.0f / 3.0f) * t2, t2, e));
+    const float a0 = frcp((0.0625f * q0) * q0), a1 = 6.0f * frcp((0.0625f * q1) * q1), a2 = frcp((0.0625f * q2) * q2);
+    const float l2 = 3.0f * a2, r0 = 3.0f * a0;
+    const float nL = fmaf(l2, fmaf(4.0f, d2, -d3), fmaf(a1, fmaf(2.0f, d2, d1), a0 * fmaf(5.0f, d1, -2.0f * d0)));
+    const float nR = fmaf(r0, fmaf(4.0f, d1, -d0), fmaf(a1, fmaf(2.0f, d1, d2), a2 * fmaf(5.0f, d2, -2.0f * d3)));
+    L = fmaf(nL, frcp(6.0f * ((a0 + a1) + l2)), v2);
+    R = fmaf(-nR, frcp(6.0f * ((a2 + a1) + r0)), v2);
 }
 
 template <typename T>

@@ -345,28 +345,23 @@ __device__ __forceinline__ float2 max2(float2 a, float2 b) { return make_float2(
 // weno5_pair (FP32 reciprocal-weight form) on two variables at once.
 __device__ __forceinline__ void weno5_pair2(float2 v0, float2 v1, float2 v2, float2 v3, float2 v4, float2 eps,
                                             float2& L, float2& R) {
-    const float2 t0 = fma2(f2(-2.f), v1, add2(v0, v2)), s0 = fma2(f2(3.f), v2, fma2(f2(-4.f), v1, v0));
-    const float2 t1 = fma2(f2(-2.f), v2, add2(v1, v3)), s1 = sub2(v1, v3);
-    const float2 t2 = fma2(f2(-2.f), v3, add2(v2, v4)), s2 = fma2(f2(3.f), v2, fma2(f2(-4.f), v3, v4));
-    const float2 q0 = fma2(mul2(f2(13.f / 12.f), t0), t0, fma2(mul2(f2(0.25f), s0), s0, eps));
-    const float2 q1 = fma2(mul2(f2(13.f / 12.f), t1), t1, fma2(mul2(f2(0.25f), s1), s1, eps));
-    const float2 q2 = fma2(mul2(f2(13.f / 12.f), t2), t2, fma2(mul2(f2(0.25f), s2), s2, eps));
-    const float2 r0 = rcp2(mul2(q0, q0)), r1 = rcp2(mul2(q1, q1)), r2 = rcp2(mul2(q2, q2));
-    // candidate polynomials times 6; the 1/6 goes into the normalisation
-    const float2 pL0 = fma2(f2(11.f), v2, fma2(f2(-7.f), v1, mul2(f2(2.f), v0)));
-    const float2 pL1 = fma2(f2(2.f), v3, fma2(f2(5.f), v2, mul2(f2(-1.f), v1)));
-    const float2 pL2 = fma2(f2(-1.f), v4, fma2(f2(5.f), v3, mul2(f2(2.f), v2)));
-    const float2 pR0 = fma2(f2(11.f), v2, fma2(f2(-7.f), v3, mul2(f2(2.f), v4)));
-    const float2 pR1 = fma2(f2(2.f), v1, fma2(f2(5.f), v2, mul2(f2(-1.f), v3)));
-    const float2 pR2 = fma2(f2(-1.f), v0, fma2(f2(5.f), v1, mul2(f2(2.f), v2)));
-    const float2 aL0 = mul2(f2(0.1f), r0), aM = mul2(f2(0.6f), r1), aL2 = mul2(f2(0.3f), r2);
-    const float2 aR0 = mul2(f2(0.1f), r2), aR2 = mul2(f2(0.3f), r0);
-    const float2 nL = fma2(aL2, pL2, fma2(aM, pL1, mul2(aL0, pL0)));
-    const float2 nR = fma2(aR2, pR2, fma2(aM, pR1, mul2(aR0, pR0)));
-    const float2 dL = mul2(f2(6.f), add2(add2(aL0, aM), aL2));
-    const float2 dR = mul2(f2(6.f), add2(add2(aR0, aM), aR2));
-    L = mul2(nL, rcp2(dL));
-    R = mul2(nR, rcp2(dR));
+    const float2 d0 = sub2(v1, v0), d1 = sub2(v2, v1), d2 = sub2(v3, v2), d3 = sub2(v4, v3);
+    const float2 t0 = sub2(d1, d0), t1 = sub2(d2, d1), t2 = sub2(d3, d2);
+    const float2 n0 = mul2(f2(-1.f), d0), n3 = mul2(f2(-1.f), d3);
+    const float2 s0 = fma2(f2(3.f), d1, n0), s1 = add2(d1, d2), s2 = fma2(f2(3.f), d2, n3);
+    const float2 e = mul2(f2(4.f), eps), k = f2(13.f / 3.f), h = f2(0.0625f);
+    const float2 q0 = fma2(s0, s0, fma2(mul2(k, t0), t0, e));
+    const float2 q1 = fma2(s1, s1, fma2(mul2(k, t1), t1, e));
+    const float2 q2 = fma2(s2, s2, fma2(mul2(k, t2), t2, e));
+    const float2 a0 = rcp2(mul2(mul2(h, q0), q0)), a2 = rcp2(mul2(mul2(h, q2), q2));
+    const float2 a1 = mul2(f2(6.f), rcp2(mul2(mul2(h, q1), q1)));
+    const float2 l2 = mul2(f2(3.f), a2), r0 = mul2(f2(3.f), a0);
+    const float2 nL = fma2(l2, fma2(f2(4.f), d2, n3),
+                           fma2(a1, fma2(f2(2.f), d2, d1), mul2(a0, fma2(f2(5.f), d1, mul2(f2(2.f), n0)))));
+    const float2 nR = fma2(r0, fma2(f2(4.f), d1, n0),
+                           fma2(a1, fma2(f2(2.f), d1, d2), mul2(a2, fma2(f2(5.f), d2, mul2(f2(2.f), n3)))));
+    L = fma2(nL, rcp2(mul2(f2(6.f), add2(add2(a0, a1), l2))), v2);
+    R = fma2(nR, rcp2(mul2(f2(-6.f), add2(add2(a2, a1), r0))), v2);
 }
 
 // Single-phase face flux on the normal axis D (HLLC, Rusanov or LF with
