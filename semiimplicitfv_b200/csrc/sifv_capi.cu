@@ -126,9 +126,11 @@ struct sifv_ctx {
     std::vector<void*> ibAllocs;
     // PCG + multigrid pressure solver (SIFV_PRESSURE_PCG_MG)
     std::vector<MgLevel> mg;
-    double* cg[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};   // x r z p q 1/m
-    double* cgScal = nullptr;    // 8 device scalars
-    double* cgPartial = nullptr; // block partial sums of the fine level
+    MgTail mgTail{};             // the levels, and the first of those that run in one block
+    double* cg[7] = {};          // x r z p q 1/m p
+    CgState* cgState = nullptr;  // scalars and the stopping flag
+    double* cgPartial = nullptr; // block partial sums of the fine level, two sums
+    int cgPrevIters = 0;         // iterations of the previous solve (first batch size)
     // mixed-precision Jacobi (semi-implicit SIFV_PREC_MIXED)
     double* mxCoef = nullptr;    // k_jacobi_coef layout, FP64
     float* mxW = nullptr;        // 2 dim FP32 weights per cell
@@ -1065,62 +1067,76 @@ int mg_alloc(sifv_ctx* c) {
     if (!c->mg.empty()) return SIFV_OK;
     int st = SIFV_OK;
     int nx = c->P.nx, ny = c->P.ny, nz = c->P.nz;
+    if (c->nint > 0x7fffffffULL) return fail(c, SIFV_ERR_UNSUPPORTED, "the PCG solver takes up to 2^31 cells");
+    std::vector<MgLevel> mg;
     for (int l = 0;; ++l) {
         MgLevel L{};
         L.nx = nx; L.ny = ny; L.nz = nz;
-        L.n = (long long)nx * ny * nz;
+        L.n = nx * ny * nz;
         L.m = dalloc(c, L.n, st);
         L.tx = dalloc(c, L.n, st);
-        L.ty = dalloc(c, L.n, st);
-        L.tz = dalloc(c, L.n, st);
+        if (c->P.dim >= 2) L.ty = dalloc(c, L.n, st);
+        if (c->P.dim >= 3) L.tz = dalloc(c, L.n, st);
         L.diag = dalloc(c, L.n, st);
-        L.r = dalloc(c, L.n, st);
-        L.t = dalloc(c, L.n, st);
+        L.iw = dalloc(c, L.n, st);
         if (l > 0) {
             L.x = dalloc(c, L.n, st);
             L.b = dalloc(c, L.n, st);
         }
         if (st != SIFV_OK) return st;
-        c->mg.push_back(L);
-        if (L.n <= 256 || (nx <= 2 && ny <= 2 && nz <= 2)) break;
+        mg.push_back(L);
+        if (L.n <= kMgCoarsest || (nx <= 2 && ny <= 2 && nz <= 2)) break;
+        if ((int)mg.size() == kMgMaxLevels) return fail(c, SIFV_ERR_UNSUPPORTED, "too many multigrid levels");
         nx = (nx > 1) ? (nx + 1) / 2 : 1;
         ny = (ny > 1) ? (ny + 1) / 2 : 1;
         nz = (nz > 1) ? (nz + 1) / 2 : 1;
     }
-    const long long n0 = c->mg[0].n;
-    for (int q = 0; q < 6; ++q) c->cg[q] = dalloc(c, n0, st);
-    c->cgScal = dalloc(c, 8, st);
-    c->cgPartial = dalloc(c, blocks(n0, kCellThreads) + 1, st);
-    return st;
+    const long long n0 = mg[0].n;
+    for (int q = 0; q < 7; ++q) c->cg[q] = dalloc(c, n0, st);
+    c->cgState = reinterpret_cast<CgState*>(dalloc(c, (sizeof(CgState) + 7) / 8, st));
+    c->cgPartial = dalloc(c, 2 * (size_t)(blocks(n0, kCellThreads) + 1), st);
+    if (st != SIFV_OK) return st;
+    mg[0].b = c->cg[1];   // the V-cycle solves M z = r
+    mg[0].x = c->cg[2];
+    MgTail& T = c->mgTail;
+    T.n = (int)mg.size();
+    T.first = 0;
+    while (T.first + 1 < T.n && mg[T.first].n > kMgTail) ++T.first;
+    for (int l = 0; l < T.n; ++l) T.l[l] = mg[l];
+    c->mg = mg;
+    return SIFV_OK;
 }
 
-constexpr double kMgOmega = 0.8;       // weighted-Jacobi relaxation
-constexpr int kMgCoarsestSweeps = 60;  // relaxation sweeps on the coarsest level
+// A kernel of a chain whose every kernel waits for the one before it
+// (grid_dep_wait): set up while that one still runs.
+template <typename... KArgs, typename... Args>
+int launch_chained(sifv_ctx* c, void (*kernel)(KArgs...), unsigned grid, unsigned threads, Args... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(grid);
+    lc.blockDim = dim3(threads);
+    lc.stream = c->stream;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    CUDA_TRY(c, cudaLaunchKernelEx(&lc, kernel, KArgs(args)...));
+    c->launches++;
+    return SIFV_OK;
+}
 
-// z = V(r): one V(1,1)-cycle from z = 0 (level 0 reads b = r, writes x = z).
-void mg_vcycle(sifv_ctx* c, int l, const double* r0, double* z0) {
-    const int dim = c->P.dim;
-    MgLevel L = c->mg[l];
-    if (l == 0) {
-        L.b = const_cast<double*>(r0);
-        L.x = z0;
-    }
-    const unsigned g = blocks(L.n, kCellThreads);
-    if (l + 1 == (int)c->mg.size()) {
-        k_mg_coarsest<<<1, 1024, 0, c->stream>>>(L, dim, kMgOmega, kMgCoarsestSweeps);
-        c->launches++;
-        return;
-    }
-    MgLevel C = c->mg[l + 1];
-    k_mg_smooth0<<<g, kCellThreads, 0, c->stream>>>(L, kMgOmega);
-    k_mg_residual<<<g, kCellThreads, 0, c->stream>>>(L, dim);
-    k_mg_restrict<<<blocks(C.n, kCellThreads), kCellThreads, 0, c->stream>>>(L, C);
-    c->launches += 3;
-    mg_vcycle(c, l + 1, nullptr, nullptr);
-    k_mg_prolong<<<g, kCellThreads, 0, c->stream>>>(L, C);
-    k_mg_smooth<<<g, kCellThreads, 0, c->stream>>>(L, dim, L.x, L.t, kMgOmega);
-    cudaMemcpyAsync(L.x, L.t, sizeof(double) * L.n, cudaMemcpyDeviceToDevice, c->stream);
-    c->launches += 2;
+// z = V(r): one V(1,1)-cycle from z = 0; r.z goes to rz[slot].
+int mg_vcycle(sifv_ctx* c, int slot) {
+    const int dim = c->P.dim, lt = c->mgTail.first;
+    int st = SIFV_OK;
+    for (int l = 0; l < lt && st == SIFV_OK; ++l)
+        st = launch_chained(c, k_mg_down, blocks(c->mg[l + 1].n, kCellThreads), kCellThreads, c->mg[l], c->mg[l + 1], dim,
+                            c->cgState);
+    if (st == SIFV_OK) st = launch_chained(c, k_mg_tail, 1, 1024, c->mgTail, dim, c->cgState, c->cgPartial, slot);
+    for (int l = lt - 1; l >= 0 && st == SIFV_OK; --l)
+        st = launch_chained(c, k_mg_up, blocks(c->mg[l].n, kCellThreads), kCellThreads, c->mg[l], c->mg[l + 1], dim,
+                            c->cgState, c->cgPartial, l == 0 ? 1 : 0, slot);
+    return st;
 }
 
 // HyprePressureSolver::solve (src/HyprePressureSolver.cpp:333-399): PCG on
@@ -1134,70 +1150,54 @@ int mg_run(sifv_ctx* c, const double* rho, const double* rhoc2, const double* rh
     st = ensure_res(c, maxIter);
     if (st != SIFV_OK) return st;
     const int dim = c->P.dim;
-    MgLevel L0 = c->mg[0];
-    const long long n0 = L0.n;
+    const int n0 = c->mg[0].n, lt = c->mgTail.first;
     const unsigned g0 = blocks(n0, kCellThreads);
-    double *x = c->cg[0], *r = c->cg[1], *z = c->cg[2], *p = c->cg[3], *q = c->cg[4], *wInv = c->cg[5];
-    double* s = c->cgScal;
+    double *x = c->cg[0], *r = c->cg[1], *z = c->cg[2], *q = c->cg[4], *wInv = c->cg[5];
+    double* p[2] = {c->cg[3], c->cg[6]};
+    CgState* S = c->cgState;
     double* part = c->cgPartial;
-    MgLevel Lf = L0;
+    MgLevel Lf = c->mg[0];
     Lf.x = x;
     Lf.b = r;   // the scaled right-hand side lands in r, then r = b - M x in place
     k_mg_fine<<<g0, kCellThreads, 0, c->stream>>>(c->P, c->F, rho, rhoc2, rhs, c->F.pA, c->ctl, Lf, wInv);
-    for (size_t l = 0; l + 1 < c->mg.size(); ++l)
+    for (int l = 0; l < lt; ++l)
         k_mg_coarsen<<<blocks(c->mg[l + 1].n, kCellThreads), kCellThreads, 0, c->stream>>>(c->mg[l], c->mg[l + 1], dim);
-    for (const MgLevel& L : c->mg) k_mg_diag<<<blocks(L.n, kCellThreads), kCellThreads, 0, c->stream>>>(L, dim);
-    // |rhs|^2 into s[4], then r = b - M x and |r/m|^2 into s[2]
-    k_mg_bnorm<<<g0, kCellThreads, 0, c->stream>>>(n0, r, wInv, part);
-    k_mg_sum<<<1, 1024, 0, c->stream>>>(part, (int)g0, s, 4);
-    Lf.b = r;
-    k_mg_residual0<<<g0, kCellThreads, 0, c->stream>>>(Lf, dim, wInv, r, part);
-    k_mg_sum<<<1, 1024, 0, c->stream>>>(part, (int)g0, s, 2);
-    c->launches += 6 + 2 * (int)c->mg.size();
+    if (lt + 1 < c->mgTail.n) k_mg_tail_setup<<<1, 1024, 0, c->stream>>>(c->mgTail, dim);
+    k_cg_start<<<g0, kCellThreads, 0, c->stream>>>(Lf, dim, wInv, r, S, part);
+    k_cg_test<<<1, 1, 0, c->stream>>>(S, tol);
+    c->launches += 4 + lt;
     LAUNCH_CHECK(c);
-    double hs[5];
-    CUDA_TRY(c, cudaMemcpyAsync(hs, s, sizeof(hs), cudaMemcpyDeviceToHost, c->stream));
-    CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-    const double bb = hs[4], eps = tol * tol;
-    double rr = hs[2];
-    int it = 0;
-    if (bb == 0.0) {   // Hypre: zero right-hand side -> zero solution
-        CUDA_TRY(c, cudaMemsetAsync(x, 0, sizeof(double) * n0, c->stream));
-        rr = 0.0;
-    } else if (!(rr <= eps * bb)) {
-        mg_vcycle(c, 0, r, z);
-        k_mg_dot<<<g0, kCellThreads, 0, c->stream>>>(n0, r, z, part);
-        k_mg_sum<<<1, 1024, 0, c->stream>>>(part, (int)g0, s, 0);
-        k_cg_direction<<<g0, kCellThreads, 0, c->stream>>>(n0, s, z, p, 1);
-        c->launches += 3;
-        while (it < maxIter) {
-            ++it;
-            k_mg_matvec_dot<<<g0, kCellThreads, 0, c->stream>>>(L0, dim, p, q, part);
-            k_mg_sum<<<1, 1024, 0, c->stream>>>(part, (int)g0, s, 1);
-            k_cg_update<<<g0, kCellThreads, 0, c->stream>>>(n0, s, x, r, p, q, wInv, part);
-            k_mg_sum<<<1, 1024, 0, c->stream>>>(part, (int)g0, s, 2);
-            c->launches += 4;
-            LAUNCH_CHECK(c);
-            CUDA_TRY(c, cudaMemcpyAsync(&hs[2], s + 2, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-            CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-            rr = hs[2];
-            if (rr <= eps * bb || !(rr == rr)) break;
-            mg_vcycle(c, 0, r, z);
-            k_mg_dot<<<g0, kCellThreads, 0, c->stream>>>(n0, r, z, part);
-            k_mg_sum<<<1, 1024, 0, c->stream>>>(part, (int)g0, s, 3);
-            k_cg_direction<<<g0, kCellThreads, 0, c->stream>>>(n0, s, z, p, 0);
-            k_cg_shift<<<1, 1, 0, c->stream>>>(s);
-            c->launches += 4;
+    // iterations in batches; the kernels queued past convergence return at once
+    CgState h{};
+    int queued = 0;
+    while (queued < maxIter) {
+        const int want = (queued == 0) ? std::max(4, c->cgPrevIters) : 3;
+        const int end = std::min(maxIter, queued + want);
+        for (int it = queued; it < end; ++it) {
+            const int slot = it & 1;
+            st = mg_vcycle(c, slot);
+            if (st == SIFV_OK)
+                st = launch_chained(c, k_cg_product, g0, kCellThreads, c->mg[0], dim, (const double*)z,
+                                    (const double*)p[slot ^ 1], p[slot], q, S, part, slot, it == 0 ? 1 : 0);
+            if (st == SIFV_OK)
+                st = launch_chained(c, k_cg_update, g0, kCellThreads, n0, x, r, (const double*)p[slot], (const double*)q,
+                                    (const double*)wInv, S, part, slot);
+            if (st != SIFV_OK) return st;
         }
+        queued = end;
+        CUDA_TRY(c, cudaMemcpyAsync(&h, S, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
+        CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+        if (h.done) break;
     }
-    k_mg_scatter<<<g0, kCellThreads, 0, c->stream>>>(c->P, Lf, c->F.pA);
+    c->cgPrevIters = h.iters;
+    k_mg_scatter<<<g0, kCellThreads, 0, c->stream>>>(c->P, Lf, c->F.pA, S);
     c->launches++;
     LAUNCH_CHECK(c);
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     // relative residual of the last iteration where the semi-implicit step looks for it
-    const double rel = (bb > 0.0) ? std::sqrt(rr / bb) : 0.0;
-    iters = it;
-    if (it > 0) std::memcpy(&c->ctlHost->res[it - 1], &rel, sizeof(double));
+    const double rel = (h.bb > 0.0) ? std::sqrt(h.rr / h.bb) : 0.0;
+    iters = h.iters;
+    if (iters > 0) std::memcpy(&c->ctlHost->res[iters - 1], &rel, sizeof(double));
     result = c->F.pA;
     mark(c, "pcg_mg");
     return SIFV_OK;
