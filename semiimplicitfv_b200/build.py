@@ -23,7 +23,7 @@ SOURCES = [("sifv_capi.cu", ["--fmad=false"]), ("sifv_noalloc.cu", ["--fmad=fals
            ("sifv_vtk.cpp", []), ("sifv_ib.cpp", ["-Xcompiler", "-ffp-contract=off"])]
 HEADERS = ["sifv_device.cuh", "sifv_common.cuh", "sifv_kernels.cuh", "sifv_sweep.cuh", "sifv_sweep_api.h",
            "sifv_ensemble.cuh", "sifv_ensemble_api.h", "sifv_adjoint.cuh", "sifv_adjoint_api.h", "sifv_dual.cuh", "sifv_march2d.cuh", "sifv_fastmath.cuh", "sifv_vtk_api.h", "sifv_ib_api.h",
-           "sifv_mg.cuh", "sifv_stage.cuh", "sifv_rn.cuh", "sifv_stage_api.h", "sifv_gs_march.cuh"]
+           "sifv_mg.cuh", "sifv_stage.cuh", "sifv_rn.cuh", "sifv_tile3d.cuh", "sifv_stage_api.h", "sifv_gs_march.cuh"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

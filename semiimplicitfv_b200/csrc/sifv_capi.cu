@@ -101,7 +101,7 @@ struct sifv_ctx {
     bool uniformAxes = false;                 // interior cell widths bitwise equal along every active axis
     int pressureKind = 0;                     // 0 Jacobi (default), 1 Gauss-Seidel
     double* gsCoef = nullptr;                 // per-cell Gauss-Seidel coefficients (2 dim + 2 arrays)
-    double* tileB[5] = {};                    // scratch states of the 2D fast and mixed stage kernel
+    double* tileB[5] = {};                    // scratch states of the 2D / 3D fast and mixed stage kernels
     double* tileC[5] = {};
     StageState stageB{}, stageC{};            // scratch states of the fused stage kernel
     bool stageReady = false;
@@ -1440,7 +1440,7 @@ bool fused_stage(const sifv_ctx* c) {
 
 // Whether the step's last stage folds the next step's dt limits into
 // ctl->dtBits.
-bool folds_dt(const sifv_ctx* c) { return (c->sweep && c->P.dim == 2) || fused_stage(c); }
+bool folds_dt(const sifv_ctx* c) { return (c->sweep && c->P.dim >= 2) || fused_stage(c); }
 
 int enqueue_dt(sifv_ctx* c, double targetDt, int useEnd) {
     const sifv_config_t& cfg = c->cfg;
@@ -1552,7 +1552,7 @@ int split_buffers(sifv_ctx* c) {
     return st;
 }
 
-// Scratch states of the 2D fast / mixed stage kernel.
+// Scratch states of the 2D and 3D fast / mixed stage kernels.
 int tile_buffers(sifv_ctx* c) {
     int st = SIFV_OK;
     for (int q = 0; q < c->P.dim + 2; ++q) {
@@ -1653,11 +1653,60 @@ int enqueue_step(sifv_ctx* c, int step, double time, double targetDt, int useEnd
                 return fail(c, SIFV_ERR_CUDA, "tile launch failed");
             }
         }
-        if (RK == 1 && tile2d_copy(c->ctl, c->tileB, U, c->ncells, c->stream, c->launches) != 0)
+        if (RK == 1 && state_copy(c->ctl, c->tileB, U, 4, c->ncells, c->stream, c->launches) != 0)
             return fail(c, SIFV_ERR_CUDA, "copy launch failed");
         launch_bc_prim(c);
         LAUNCH_CHECK(c);
         c->dtReady = cfg.constDt <= 0 && c->forcedDt <= 0;
+        return SIFV_OK;
+    }
+    if (c->sweep && P.dim == 3) {
+        double* U[5] = {c->F.rho, c->F.rhoU, c->F.rhoV, c->F.rhoW, c->F.rhoE};
+        const int RK = cfg.RKOrder;
+        const bool fold = cfg.constDt <= 0 && c->forcedDt <= 0;
+        for (int s = 0; s < RK; ++s) {
+            StageCoef K{};
+            rk_coef(RK, s, K);
+            Tile3Args T{};
+            T.P = c->P;
+            T.C.gamma = c->P.gamma;
+            T.C.pInf = c->P.pInf;
+            T.C.invGm1 = 1.0 / (c->P.gamma - 1.0);
+            T.C.gPinf = c->P.gamma * c->P.pInf;
+            T.eps = cfg.wenoEps;
+            T.ctl = c->ctl;
+            T.a1 = K.c1 / K.c4;
+            T.a2 = K.c2 / K.c4;
+            T.a3 = K.c3 / K.c4;
+            for (int d = 0; d < 3; ++d) T.inv[d] = c->invW[d];
+            T.dx = c->F.dx;
+            T.dy = c->F.dy;
+            T.dz = c->F.dz;
+            T.last = (s == RK - 1) ? 1 : 0;
+            T.dtNext = (T.last && fold) ? 1 : 0;
+            T.cfl = cfg.cfl;
+            T.velU = c->F.velU;
+            T.velV = c->F.velV;
+            T.velW = c->F.velW;
+            T.pres = c->F.pres;
+            double* const* in = (s == 0) ? U : (s == 1) ? c->tileB : c->tileC;
+            double* const* out = (RK > 1 && s == RK - 1) ? U : (s == 0) ? c->tileB : c->tileC;
+            for (int q = 0; q < 5; ++q) {
+                T.in[q] = in[q];
+                T.out[q] = out[q];
+                T.u0[q] = (s > 0 && K.c2 != 0.0) ? U[q] : nullptr;
+            }
+            if (tile3d_stage(T, c->stream, cfg.precision == SIFV_PREC_MIXED, c->launches,
+                             c->profiling ? mark_cb : nullptr, c) != 0) {
+                LAUNCH_CHECK(c);
+                return fail(c, SIFV_ERR_CUDA, "tile launch failed");
+            }
+        }
+        if (RK == 1 && state_copy(c->ctl, c->tileB, U, 5, c->ncells, c->stream, c->launches) != 0)
+            return fail(c, SIFV_ERR_CUDA, "copy launch failed");
+        launch_bc_prim(c);
+        LAUNCH_CHECK(c);
+        c->dtReady = fold;
         return SIFV_OK;
     }
     if (c->sweep) {
@@ -2014,12 +2063,12 @@ int sifv_create(const sifv_config_t* cfg, const sifv_mesh_t* mesh, int device, s
     F.dx = g[0]; F.dy = g[1]; F.dz = g[2]; F.adx2 = g[3]; F.ady2 = g[4]; F.adz2 = g[5];
     if (cfg->precision != SIFV_PREC_FP64 && !cfg->semiImplicit) {
         c->sweep = true;
-        c->rhoP = dalloc(c, n, st);
-        c->rhsBuf[0] = dalloc(c, n, st);
-        c->rhsBuf[1] = dalloc(c, n, st);
-        if (dim >= 2) c->rhsBuf[2] = dalloc(c, n, st);
-        if (dim >= 3) c->rhsBuf[3] = dalloc(c, n, st);
-        c->rhsBuf[4] = dalloc(c, n, st);
+        if (dim == 1) {
+            c->rhoP = dalloc(c, n, st);
+            c->rhsBuf[0] = dalloc(c, n, st);
+            c->rhsBuf[1] = dalloc(c, n, st);
+            c->rhsBuf[4] = dalloc(c, n, st);
+        }
         const std::vector<double>* w[3] = {&dxv, &dyv, &dzv};
         for (int a = 0; a < 3; ++a) {
             std::vector<double> inv(w[a]->size());
@@ -2032,7 +2081,7 @@ int sifv_create(const sifv_config_t* cfg, const sifv_mesh_t* mesh, int device, s
         if (st == SIFV_OK) cudaStreamSynchronize(c->stream);   // host vectors above go out of scope
     }
     if (st == SIFV_OK) st = ensure_res(c, std::max(cfg->maxPressureIters, 1));
-    if (st == SIFV_OK) st = fused_stage(c) ? stage_buffers(c) : (c->sweep && dim == 2) ? tile_buffers(c) : split_buffers(c);
+    if (st == SIFV_OK) st = fused_stage(c) ? stage_buffers(c) : (c->sweep && dim >= 2) ? tile_buffers(c) : split_buffers(c);
     if (st == SIFV_OK) {
         cudaError_t e = cudaStreamSynchronize(c->stream);
         if (e != cudaSuccess) st = fail(c, SIFV_ERR_CUDA, cudaGetErrorString(e));

@@ -10,60 +10,32 @@
 #include "sifv_sweep.cuh"
 #include "sifv_sweep_api.h"
 #include "sifv_march2d.cuh"
+#include "sifv_tile3d.cuh"
 
 namespace sifv {
 
 namespace {
 
-constexpr int kSegment = 32;    // cells per thread along y / z
 constexpr int kSegmentX = 510;  // cells per warp along x: 16 steps of 32 positions
 
-template <int DIM, typename T>
-int stage_dim(const SweepArgs& A, cudaStream_t s, int& launches, LaunchMark mark, void* user) {
+template <typename T>
+int stage_1d(const SweepArgs& A, cudaStream_t s, int& launches, LaunchMark mark, void* user) {
     const Params& P = A.P;
-    {
-        long long warps = (long long)P.ny * P.nz * ((P.nx + A.segx - 1) / A.segx);
-        unsigned g = (unsigned)((warps + 3) / 4);
-        k_sweep_x<DIM, T><<<g, 128, 0, s>>>(A);
-        ++launches;
-        if (mark) mark(user, "sweep_x");
-    }
-    if (DIM == 1) {
-        long long n = (long long)P.nx;
-        k_rk_update<DIM><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(A);
-        ++launches;
-        if (mark) mark(user, "rk_update");
-    } else {
-        dim3 g1((P.nx + 127) / 128, (P.ny + A.seg - 1) / A.seg, P.nz);
-        k_sweep_line<1, DIM, T, DIM == 2><<<g1, 128, 0, s>>>(A);
-        ++launches;
-        if (mark) mark(user, "sweep_y");
-        if (DIM == 3) {
-            dim3 g2((P.nx + 127) / 128, (P.nz + A.seg - 1) / A.seg, P.ny);
-            k_sweep_line<2, DIM, T, true><<<g2, 128, 0, s>>>(A);
-            ++launches;
-            if (mark) mark(user, "sweep_z");
-        }
-    }
+    long long warps = (P.nx + A.segx - 1) / A.segx;
+    k_sweep_x<1, T><<<(unsigned)((warps + 3) / 4), 128, 0, s>>>(A);
+    ++launches;
+    if (mark) mark(user, "sweep_x");
+    k_rk_update<1><<<(unsigned)(((long long)P.nx + 255) / 256), 256, 0, s>>>(A);
+    ++launches;
+    if (mark) mark(user, "rk_update");
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
 }  // namespace
 
 int sweep_stage(SweepArgs A, cudaStream_t s, bool mixed, int& launches, LaunchMark mark, void* user) {
-    A.seg = kSegment;
     A.segx = kSegmentX;
-    switch (A.P.dim) {
-        case 1:
-            return mixed ? stage_dim<1, float>(A, s, launches, mark, user)
-                         : stage_dim<1, double>(A, s, launches, mark, user);
-        case 2:
-            return mixed ? stage_dim<2, float>(A, s, launches, mark, user)
-                         : stage_dim<2, double>(A, s, launches, mark, user);
-        default:
-            return mixed ? stage_dim<3, float>(A, s, launches, mark, user)
-                         : stage_dim<3, double>(A, s, launches, mark, user);
-    }
+    return mixed ? stage_1d<float>(A, s, launches, mark, user) : stage_1d<double>(A, s, launches, mark, user);
 }
 
 namespace {
@@ -134,16 +106,79 @@ int tile2d_stage(const TileArgs& A, cudaStream_t s, bool mixed, int& launches, L
     return st;
 }
 
-int tile2d_copy(const Ctl* ctl, const double* const in[4], double* const out[4], size_t n, cudaStream_t s,
-                int& launches) {
-    Copy4 C;
-    for (int q = 0; q < 4; ++q) {
+int state_copy(const Ctl* ctl, const double* const* in, double* const* out, int count, size_t n, cudaStream_t s,
+               int& launches) {
+    CopyN C{};
+    C.count = count;
+    for (int q = 0; q < count; ++q) {
         C.src[q] = in[q];
         C.dst[q] = out[q];
     }
-    k_copy4<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(ctl, C, n);
+    k_copy_state<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(ctl, C, n);
     ++launches;
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+namespace {
+
+template <typename T, int RS>
+int tile3_launch(Tile3Args A, cudaStream_t s) {
+    constexpr size_t bytes = Tile3::smem<T>();
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    if (cudaFuncSetAttribute(k_tile3d<T, RS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return -1;
+    A.tilesX = (A.P.nx + Tile3::TX - 1) / Tile3::TX;
+    A.tilesY = (A.P.ny + Tile3::TY - 1) / Tile3::TY;
+    // Segments along z: the walk of a segment costs its planes and about
+    // three planes' worth of start-up, and the blocks run in waves of two per
+    // SM; take the segment count with the shortest sum (down to one plane: a
+    // small mesh is one wave, as long as its longest walk).
+    const long long tiles = (long long)A.tilesX * A.tilesY, slots = 2LL * sms;
+    double best = 0.0;
+    A.segs = 1;
+    for (int g = 1; g <= A.P.nz && g <= 64; ++g) {
+        const int planes = (A.P.nz + g - 1) / g;
+        const double cost = (double)((tiles * g + slots - 1) / slots) * (planes + 3);
+        if (g == 1 || cost < best) {
+            best = cost;
+            A.segs = g;
+        }
+    }
+    A.segPlanes = (A.P.nz + A.segs - 1) / A.segs;
+    A.segs = (A.P.nz + A.segPlanes - 1) / A.segPlanes;
+    const long long grid = tiles * A.segs;
+    if (grid > 0x7fffffffLL) return -1;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3((unsigned)grid);
+    lc.blockDim = dim3(Tile3::threads);
+    lc.dynamicSmemBytes = bytes;
+    lc.stream = s;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    return cudaLaunchKernelEx(&lc, k_tile3d<T, RS>, A) == cudaSuccess ? 0 : -1;
+}
+
+template <typename T>
+int tile3_dispatch(const Tile3Args& A, cudaStream_t s) {
+    switch (A.P.riemann) {
+        case SIFV_HLLC: return tile3_launch<T, SIFV_HLLC>(A, s);
+        case SIFV_RUSANOV: return tile3_launch<T, SIFV_RUSANOV>(A, s);
+        default: return tile3_launch<T, SIFV_LF>(A, s);
+    }
+}
+
+}  // namespace
+
+int tile3d_stage(const Tile3Args& A, cudaStream_t s, bool mixed, int& launches, LaunchMark mark, void* user) {
+    const int st = mixed ? tile3_dispatch<float>(A, s) : tile3_dispatch<double>(A, s);
+    ++launches;
+    if (mark) mark(user, "tile3d");
+    return st;
 }
 
 namespace {

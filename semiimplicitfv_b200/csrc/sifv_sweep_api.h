@@ -30,7 +30,6 @@ struct SweepArgs {
     FluxConsts C;
     RKUpdate K;
     double eps;
-    int seg;       // cells per thread segment (line sweeps)
     int segx;      // cells per warp segment of a row (x sweep), 32 m - 2
     double* rhs[5];  // FP64 rhs buffer (rho, rhoU, rhoV, rhoW, rhoE)
     double* rhoP;    // stage primitive density: the conservative rho is updated in place by the
@@ -62,20 +61,42 @@ struct TileArgs {
     const double *dx, *dy;      // cell widths (ghosts included)
 };
 
+// One RK stage of the 3D explicit step as one fused kernel
+// (sifv_tile3d.cuh), as TileArgs.
+struct Tile3Args {
+    Params P;
+    FluxConsts C;
+    double eps;
+    Ctl* ctl;
+    const double* in[5];    // stage input: rho, rhoU, rhoV, rhoW, rhoE
+    const double* u0[5];    // step-start state (own cells), null when a2 == 0
+    double* out[5];         // stage output (u0 or scratch, never `in`)
+    double a1, a2, a3;
+    const double* inv[3];   // 1 / d per cell (ghosts included)
+    const double *dx, *dy, *dz;
+    int last;               // write the primitives of the new state
+    int dtNext;             // ... and fold its acoustic dt into ctl->dtBits
+    double cfl;
+    double *velU, *velV, *velW, *pres;
+    int tilesX, tilesY, segs, segPlanes;   // set by the launcher
+};
+
 // Called after each kernel launch with the kernel family's name (per-kernel
 // timing); may be null.
 typedef void (*LaunchMark)(void* user, const char* family);
 
-// One RK stage of the explicit step on the fused sweep kernels
+// One RK stage of the 1D explicit step on the fused sweep kernels
 // (mixed: FP32 reconstruction / Riemann bulk).  Returns 0 on success.
 int sweep_stage(SweepArgs A, cudaStream_t s, bool mixed, int& launches, LaunchMark mark = nullptr,
                 void* user = nullptr);
 
 int tile2d_stage(const TileArgs& A, cudaStream_t s, bool mixed, int& launches, LaunchMark mark = nullptr,
                  void* user = nullptr);
-// out[q] = in[q] over n values, skipped when the step is (device-side loops).
-int tile2d_copy(const Ctl* ctl, const double* const in[4], double* const out[4], size_t n, cudaStream_t s,
-                int& launches);
+int tile3d_stage(const Tile3Args& A, cudaStream_t s, bool mixed, int& launches, LaunchMark mark = nullptr,
+                 void* user = nullptr);
+// out[q] = in[q], q < count, over n values, skipped when the step is (device-side loops).
+int state_copy(const Ctl* ctl, const double* const* in, double* const* out, int count, size_t n, cudaStream_t s,
+               int& launches);
 
 // End-of-step conservative -> primitive on interior cells.
 int sweep_finish_prim(const Params& P, const Fields& F, const Ctl* ctl, cudaStream_t s, int& launches);

@@ -16,8 +16,8 @@ EDGES = [3, 4, 25, 26, 27, 51, 52, 53, 79]
 @pytest.mark.parametrize("rk,block", [(1, 32), (2, 64), (3, 512)])
 def test_strip_edges_match_the_oracle(bc, rk, block):
     cfg = abi.config_defaults(dim=1, nGhost=3, RKOrder=rk, reconOrder=abi.WENO5, cfl=0.5, maxDt=1.0)
-    # domains from 0, where the last node is the upper end exactly (the ensemble is given the ends, the oracle the nodes)
-    inst = [_tube(cfg, n, 0.0, 1.0 + 0.1 * k, (1.0 + 0.1 * k, 0.05 * (k % 3), 1.0 + 0.2 * k),
+    # on [0, 1], whose last node is the upper end exactly (the ensemble is given the ends, the oracle the nodes)
+    inst = [_tube(cfg, n, 0.0, 1.0, (1.0 + 0.1 * k, 0.05 * (k % 3), 1.0 + 0.2 * k),
                   (0.125, -0.02 * (k % 2), 0.1), bc) for k, n in enumerate(EDGES)]
     ens = _ensemble(inst)
     t, s, _ = ens.run(0.02, 0, block)
