@@ -19,7 +19,9 @@
 // the FP64 pipe is 61 % busy at 1024^2 (207 us per stage), held there by
 // barriers and load latency at three blocks per SM.  Per RK3 step, the
 // separate kernels against this one: 1D 1000 cells 82 -> 26 us; 256^2
-// 134 -> 92; 1531 x 1021 viscous 1370 -> 1000; 480 x 352 two-phase 320 -> 278.
+// 134 -> 92; 1531 x 1021 viscous 1370 -> 1000; 480 x 352 two-phase 320 -> 262
+// (278 with the fluxes in a buffer of their own, which leaves room for two
+// two-phase blocks per SM instead of three).
 #pragma once
 
 #include "sifv_stage_api.h"
@@ -44,8 +46,8 @@ struct StageTile {
     static constexpr int R = (DIM == 1 || RX > RY) ? RX : RY;
     static constexpr int FX = (TX + 1) * TY, FY = (DIM == 1) ? 0 : TX * (TY + 1);
     static constexpr int NF = DIM + 2 + (NPH > 0 ? 1 + 2 * NPH : 0);   // flux slots
-    static constexpr size_t smem = ((size_t)(NV + NPH) * W * H + 2 * (size_t)NV * R + (size_t)NF * (FX + FY)) *
-                                   sizeof(double);
+    static constexpr size_t smem = ((size_t)(NV + NPH) * W * H + 2 * (size_t)NV * R) * sizeof(double);
+    static_assert(NF <= 2 * NV, "a face's fluxes take the place of the values it read");
     static_assert((DIM + 1) * (FX + FY) <= 2 * NV * R, "the face stresses reuse the reconstruction buffer");
 };
 
@@ -119,13 +121,15 @@ __device__ __forceinline__ void stage_recon(const Params& P, const double* sW, d
     }
 }
 
-// Riemann problems of direction d's faces into sF (slot-major).  Both
+// Riemann problems of direction d's faces.  A face's fluxes take the place of
+// the values only it reads: slots 0 .. NV - 1 of its left cell's high-face
+// values, the rest of its right cell's low-face ones (stage_flux).  Both
 // directions run the axis-0 solver on (normal, transverse) components: in two
 // dimensions its sums over the components are commutative, so exchanging the
 // components changes no bit.
 template <int DIM, int NPH, int RS>
-__device__ __forceinline__ void stage_faces(int d, const Params& P, const double* sW, const double* sHi,
-                                            const double* sLo, double* sF, int lx, int ly) {
+__device__ __forceinline__ void stage_faces(int d, const Params& P, const double* sW, double* sHi, double* sLo, int lx,
+                                            int ly) {
     using T = StageTile<DIM, NPH>;
     const int gx = T::TX + (d == 0), nface = (d == 0) ? T::FX : T::FY;
     const int cx = T::TX + (d == 0 ? 2 : 0), R_ = T::R;
@@ -167,12 +171,15 @@ __device__ __forceinline__ void stage_faces(int d, const Params& P, const double
         }
         FaceFlux<NPH> Fx;
         stage_riemann<NPH, RS>(P, L, R, Fx);
-        sF[t] = Fx.mass;
+        auto put = [&](int q, double x) {
+            if (q < NV) sHi[q * R_ + cl] = x; else sLo[(q - NV) * R_ + cr] = x;
+        };
+        put(0, Fx.mass);
 #pragma unroll
-        for (int q = 0; q < DIM; ++q) sF[((DIM == 1) ? 1 : 1 + (q ^ d)) * nface + t] = Fx.mom[q];
-        sF[(DIM + 1) * nface + t] = Fx.energy;
+        for (int q = 0; q < DIM; ++q) sHi[((DIM == 1) ? 1 : 1 + (q ^ d)) * R_ + cl] = Fx.mom[q];
+        put(DIM + 1, Fx.energy);
         if (NPH > 0) {
-            sF[(DIM + 2) * nface + t] = Fx.fvel;
+            put(DIM + 2, Fx.fvel);
             // upwinded partial-density flux (src/ExplicitSolver.cpp:307-326)
             const int right = (i + 3) + ((DIM == 1) ? 0 : (j + 3) * T::W);
             const int upw = (Fx.mass >= 0) ? right - ((d == 0) ? 1 : T::W) : right;
@@ -180,11 +187,42 @@ __device__ __forceinline__ void stage_faces(int d, const Params& P, const double
 #pragma unroll
             for (int ph = 0; ph < NPH; ++ph) {
                 if (ph < P.nPh) {
-                    sF[(DIM + 3 + ph) * nface + t] = Fx.alpha[ph];
-                    sF[(DIM + 3 + NPH + ph) * nface + t] = (sW[(NV + ph) * (T::W * T::H) + upw] / rhoUpw) * Fx.mass;
+                    put(DIM + 3 + ph, Fx.alpha[ph]);
+                    put(DIM + 3 + NPH + ph, (sW[(NV + ph) * (T::W * T::H) + upw] / rhoUpw) * Fx.mass);
                 }
             }
         }
+    }
+}
+
+// Flux slot q of the face whose left cell is reconstructed cell cl of
+// direction D.
+template <int D, int DIM, int NPH>
+__device__ __forceinline__ double stage_flux(const double* sHi, const double* sLo, int q, int cl) {
+    using T = StageTile<DIM, NPH>;
+    return (q < T::NV) ? sHi[q * T::R + cl] : sLo[(q - T::NV) * T::R + cl + ((D == 0) ? 1 : T::TX)];
+}
+
+// One direction's share of the cell's divergence, slot by slot (div_slot's
+// and div_fvel's order): r of every slot, starting from 0 along x.
+template <int D, int DIM, int NPH>
+__device__ __forceinline__ void stage_div(const Params& P, const double* sHi, const double* sLo, int i, int j, double c,
+                                          double* r) {
+    using T = StageTile<DIM, NPH>;
+    const int lo = (D == 0) ? i + (T::TX + 2) * j : i + T::TX * j, hi = lo + ((D == 0) ? 1 : T::TX);
+#pragma unroll
+    for (int q = 0; q < T::NF; ++q) {
+        if (NPH > 0 && q == 0) continue;   // the mixture density is the sum of the partial densities
+        const double fl = c * stage_flux<D, DIM, NPH>(sHi, sLo, q, lo), fh = c * stage_flux<D, DIM, NPH>(sHi, sLo, q, hi);
+        double x = (D == 0) ? 0.0 : r[q];
+        if (NPH > 0 && q == DIM + 2) {   // the face velocity: the opposite signs
+            x -= fl;
+            x += fh;
+        } else {
+            x += fl;
+            x -= fh;
+        }
+        r[q] = x;
     }
 }
 
@@ -270,7 +308,7 @@ __device__ __noinline__ void stage_ghosts(const StageArgs& A, int i, int j, doub
 }
 
 template <int DIM, int NPH, int RS>
-__global__ void __launch_bounds__(StageTile<DIM, NPH>::threads, (DIM == 2 && NPH == 0) ? 3 : 2)
+__global__ void __launch_bounds__(StageTile<DIM, NPH>::threads, 3)
     k_stage(const __grid_constant__ StageArgs A) {
     using T = StageTile<DIM, NPH>;
     constexpr int NV = T::NV, WH = T::W * T::H;
@@ -278,7 +316,6 @@ __global__ void __launch_bounds__(StageTile<DIM, NPH>::threads, (DIM == 2 && NPH
     double* const sW = sm;                       // primitives, then the partial densities
     double* const sHi = sW + (NV + NPH) * WH;    // high- / low-face values of the direction at hand
     double* const sLo = sHi + NV * T::R;
-    double* const sF = sLo + NV * T::R;          // x face fluxes, then y
     const Params& P = A.P;
     const int i0 = (int)blockIdx.x * T::TX, j0 = (int)blockIdx.y * T::TY;
     const int lx = min(T::TX, P.nx - i0), ly = (DIM == 1) ? 1 : min(T::TY, P.ny - j0);   // cells of this tile
@@ -316,60 +353,51 @@ __global__ void __launch_bounds__(StageTile<DIM, NPH>::threads, (DIM == 2 && NPH
     __syncthreads();
 
     // ---- fluxes ----
-#pragma unroll 1
-    for (int d = 0; d < DIM; ++d) {
-        if (d == 0) stage_recon<0, DIM, NPH>(P, sW, sHi, sLo, lx, ly);
-        else if (DIM >= 2) stage_recon<(DIM >= 2) ? 1 : 0, DIM, NPH>(P, sW, sHi, sLo, lx, ly);
+    // divergence (k_assemble's accumulation order: x low face, x high face, y ...)
+    const int i = (int)threadIdx.x % T::TX, j = (int)threadIdx.x / T::TX;
+    const bool mine = i < lx && j < ly;
+    double f[T::NF];
+    stage_recon<0, DIM, NPH>(P, sW, sHi, sLo, lx, ly);
+    __syncthreads();
+    stage_faces<DIM, NPH, RS>(0, P, sW, sHi, sLo, lx, ly);
+    __syncthreads();
+    const double dxi = mine ? A.dx[i0 + i + P.ngx] : 1.0, dyj = mine ? A.dy[j0 + j + P.ngy] : 1.0, dzk = A.dz[0];
+    const double vol = dxi * dyj * dzk;
+    const double cx = (dyj * dzk) / vol, cy = (DIM >= 2) ? (dxi * dzk) / vol : 0.0;
+    if (mine) stage_div<0, DIM, NPH>(P, sHi, sLo, i, j, cx, f);
+    if (DIM >= 2) {
+        constexpr int D1 = (DIM >= 2) ? 1 : 0;
         __syncthreads();
-        stage_faces<DIM, NPH, RS>(d, P, sW, sHi, sLo, sF + d * (T::NF * T::FX), lx, ly);
+        stage_recon<D1, DIM, NPH>(P, sW, sHi, sLo, lx, ly);
         __syncthreads();
+        stage_faces<DIM, NPH, RS>(1, P, sW, sHi, sLo, lx, ly);
+        __syncthreads();
+        if (mine) stage_div<D1, DIM, NPH>(P, sHi, sLo, i, j, cy, f);
     }
-    double* const sV = sHi;   // face stresses in place of the reconstructed values
+    double* const sV = sHi;   // face stresses in place of the fluxes
     if (P.visc) {
+        __syncthreads();
         stage_visc<0, DIM, NPH>(A, sW, sV, i0, j0, lx, ly);
         if (DIM >= 2) stage_visc<(DIM >= 2) ? 1 : 0, DIM, NPH>(A, sW, sV + (DIM + 1) * T::FX, i0, j0, lx, ly);
         __syncthreads();
     }
 
-    // ---- divergence (k_assemble's accumulation order) and update ----
+    // ---- update ----
     double dtLimit = __longlong_as_double(0x7ff0000000000000LL);
-    const int i = (int)threadIdx.x % T::TX, j = (int)threadIdx.x / T::TX;
-    if (i < lx && j < ly) {
+    if (mine) {
         const size_t c = cidx(P, i0 + i, j0 + j, 0);
         const int w = (i + 3) + ((DIM == 1) ? 0 : (j + 3) * T::W);
-        const double dxi = A.dx[i0 + i + P.ngx], dyj = A.dy[j0 + j + P.ngy], dzk = A.dz[0];
-        const double vol = dxi * dyj * dzk;
-        const double cx = (dyj * dzk) / vol, cy = (DIM >= 2) ? (dxi * dzk) / vol : 0.0;
-        const double* fx = sF + i + (T::TX + 1) * j;
-        const double* fy = sF + T::NF * T::FX + i + T::TX * j;
-        auto div = [&](int slot) {
-            double r = 0.0;
-            r += cx * fx[slot * T::FX];
-            r -= cx * fx[slot * T::FX + 1];
-            if (DIM >= 2) {
-                r += cy * fy[slot * T::FY];
-                r -= cy * fy[slot * T::FY + T::TX];
-            }
-            return r;
-        };
         double r[DIM + 2];
 #pragma unroll
-        for (int q = 0; q < DIM + 2; ++q) r[q] = div(q);
+        for (int q = 0; q < DIM + 2; ++q) r[q] = (NPH > 0 && q == 0) ? 0.0 : f[q];
         double rAR[NPH > 0 ? NPH : 1], rA[NPH > 0 ? NPH : 1];
         if (NPH > 0) {
-            constexpr int FV = DIM + 2;
-            double divU = 0.0;
-            divU -= cx * fx[FV * T::FX];
-            divU += cx * fx[FV * T::FX + 1];
-            if (DIM >= 2) {
-                divU -= cy * fy[FV * T::FY];
-                divU += cy * fy[FV * T::FY + T::TX];
-            }
+            const double divU = f[DIM + 2 < T::NF ? DIM + 2 : 0];
 #pragma unroll
             for (int ph = 0; ph < NPH; ++ph) {
                 if (ph < P.nPh) {
-                    rAR[ph] = div(DIM + 3 + NPH + ph);
-                    rA[ph] = div(DIM + 3 + ph);
+                    rAR[ph] = f[DIM + 3 + NPH + ph];
+                    rA[ph] = f[DIM + 3 + ph];
                     rA[ph] += sW[(DIM + 2 + ph) * WH + w] * divU;
                 }
             }
