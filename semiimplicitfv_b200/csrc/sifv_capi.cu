@@ -139,6 +139,7 @@ struct sifv_ctx {
     int lastInPlace = 0;         // the last pressure solve left its result in F.pA
     int jacPrevIters = 0;        // iterations of the previous Jacobi solve (first batch size)
     unsigned jacGrid = 0;        // resident-grid size of the grid-stride Jacobi kernels
+    int jacSms = 0;              // SMs (segments of the paired iterations)
     unsigned mxGrid = 0;         // the same for k_mx_sweep
     int adjFp32 = 0;             // FP32 local Jacobians in the reverse sweep
 };
@@ -551,6 +552,29 @@ int igr_solve(sifv_ctx* c, int step) {
     return SIFV_OK;
 }
 
+// A kernel of a chain whose every kernel waits for the one before it
+// (grid_dep_wait): set up while that one still runs.
+template <typename... KArgs, typename... Args>
+int launch_chained_smem(sifv_ctx* c, void (*kernel)(KArgs...), dim3 grid, unsigned threads, size_t smem, Args... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = grid;
+    lc.blockDim = dim3(threads);
+    lc.dynamicSmemBytes = smem;
+    lc.stream = c->stream;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    CUDA_TRY(c, cudaLaunchKernelEx(&lc, kernel, KArgs(args)...));
+    c->launches++;
+    return SIFV_OK;
+}
+template <typename... KArgs, typename... Args>
+int launch_chained(sifv_ctx* c, void (*kernel)(KArgs...), dim3 grid, unsigned threads, Args... args) {
+    return launch_chained_smem(c, kernel, grid, threads, 0, args...);
+}
+
 // Jacobi iterations on (rho, rhoc2, rhs) with initial guess in F.pA;
 // returns the number of iterations as JacobiPressureSolver::solve does and
 // the buffer holding the result.
@@ -580,63 +604,100 @@ int jacobi_run(sifv_ctx* c, const double* rho, const double* rhoc2, const double
         CUDA_TRY(c, cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, c->device));
         CUDA_TRY(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb1, k_jacobi_face, kCellThreads, 0));
         CUDA_TRY(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb2, k_jacobi_pre, kCellThreads, 0));
+        c->jacSms = sm;
         c->jacGrid = (unsigned)std::max(1, sm * std::max(1, std::min(nb1, nb2)));
     }
     const unsigned gj = std::min(g, c->jacGrid);
+    const Params& P = c->P;
+    const dim3 g3((unsigned)((P.nx + 31) / 32), (unsigned)((P.ny + 7) / 8), (unsigned)((P.nz + kJacZ - 1) / kJacZ));
+    // 3D: two iterations per launch, except with a decomposed mesh, whose
+    // ghost layers and residual are exchanged between the iterations.  The
+    // walk of a segment costs its planes and about three more, and the blocks
+    // run in waves of one per SM: the segment count with the shortest sum.
+    const bool pairs = P.dim == 3 && !c->exchangeFaces;
+    dim3 gp((unsigned)((P.nx + 31) / 32), (unsigned)((P.ny + kJac2Y - 1) / kJac2Y), 1);
+    int planes = P.nz;
+    if (pairs) {
+        const long long tiles = (long long)gp.x * gp.y, slots = std::max(1, c->jacSms);
+        double best = 0.0;
+        for (int s = 1; s <= P.nz && s <= 64; ++s) {
+            const int n = (P.nz + s - 1) / s;
+            const double cost = (double)((tiles * s + slots - 1) / slots) * (n + 3);
+            if (s == 1 || cost < best) {
+                best = cost;
+                planes = n;
+            }
+        }
+        gp.z = (unsigned)((P.nz + planes - 1) / planes);
+        CUDA_TRY(c, cudaFuncSetAttribute(faceCoef ? k_jacobi3_pair<true> : k_jacobi3_pair<false>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(faceCoef ? jac2_smem<true>() : jac2_smem<false>())));
+    }
+    double* const buf[2] = {c->F.pA, c->F.pB};
+    int launched = 0;   // an iteration or a pair reads buf[launched % 2] and writes the other
+    auto single = [&](int n, const double* pin, double* pout) {
+        if (P.dim == 3)
+            return launch_chained(c, faceCoef ? k_jacobi3<true> : k_jacobi3<false>, g3, 256, P,
+                                  (const double*)c->jacCoef, c->ncells, rhoc2, rhs, pin, pout, c->ctl, n, tol);
+        if (faceCoef)
+            return launch_chained(c, k_jacobi_face, dim3(gj), kCellThreads, P, (const double*)c->jacCoef, c->ncells, rhoc2,
+                                  rhs, pin, pout, c->ctl, n, tol);
+        return launch_chained(c, k_jacobi_pre, dim3(gj), kCellThreads, P, (const double*)c->jacCoef, c->ncells, rhs, pin,
+                              pout, c->ctl, n, tol);
+    };
     int it = 0, batch = c->jacPrevIters > 5 ? (3 * c->jacPrevIters) / 4 : 4;
     bool first = true;
     int done = 0;
     while (it < maxIter) {
-        int nb = std::min(batch, maxIter - it);
-        for (int q = 0; q < nb; ++q, ++it) {
-            const double* pin = (it & 1) ? c->F.pB : c->F.pA;
-            double* pout = (it & 1) ? c->F.pA : c->F.pB;
-            {   // decomposed mesh: the iterate's ghost layers from the neighbours (src/JacobiPressureSolver.cpp:72)
-                int st = exchange_scalar(c, pin);
+        const int from = it, end = std::min(it + batch + (pairs ? batch & 1 : 0), maxIter);
+        while (it < end) {
+            const double* pin = buf[launched & 1];
+            double* pout = buf[(launched & 1) ^ 1];
+            if (pairs && it + 2 <= end) {
+                st = launch_chained_smem(c, faceCoef ? k_jacobi3_pair<true> : k_jacobi3_pair<false>, gp, kJac2Threads,
+                                         faceCoef ? jac2_smem<true>() : jac2_smem<false>(), P, (const double*)c->jacCoef,
+                                         c->ncells, rhoc2, rhs, pin, pout, c->ctl, it, tol, planes);
                 if (st != SIFV_OK) return st;
-            }
-            if (c->P.dim == 3) {
-                const dim3 g3((unsigned)((c->P.nx + 31) / 32), (unsigned)((c->P.ny + 7) / 8),
-                              (unsigned)((c->P.nz + kJacZ - 1) / kJacZ));
-                if (faceCoef)
-                    k_jacobi3<true><<<g3, 256, 0, c->stream>>>(c->P, c->jacCoef, c->ncells, rhoc2, rhs, pin, pout,
-                                                               c->ctl, it, tol);
-                else
-                    k_jacobi3<false><<<g3, 256, 0, c->stream>>>(c->P, c->jacCoef, c->ncells, rhoc2, rhs, pin, pout,
-                                                                c->ctl, it, tol);
-            } else if (faceCoef)
-                k_jacobi_face<<<gj, kCellThreads, 0, c->stream>>>(c->P, c->jacCoef, c->ncells, rhoc2, rhs, pin, pout,
-                                                                 c->ctl, it, tol);
-            else
-                k_jacobi_pre<<<gj, kCellThreads, 0, c->stream>>>(c->P, c->jacCoef, c->ncells, rhs, pin, pout, c->ctl,
-                                                                it, tol);
-            {   // the iteration's change, maximum over the ranks, before the next iteration tests it
-                int st = reduce_residual(c, &c->ctl->res[it]);
+                it += 2;
+            } else {
+                // decomposed mesh: the iterate's ghost layers from the neighbours (src/JacobiPressureSolver.cpp:72)
+                st = exchange_scalar(c, pin);
+                if (st == SIFV_OK) st = single(it, pin, pout);
+                // the iteration's change, maximum over the ranks, before the next iteration tests it
+                if (st == SIFV_OK) st = reduce_residual(c, &c->ctl->res[it]);
                 if (st != SIFV_OK) return st;
+                ++it;
             }
+            ++launched;
         }
-        c->launches += nb;
         LAUNCH_CHECK(c);
         CUDA_TRY(c, cudaMemcpyAsync(c->ctlHost, c->ctl, sizeof(Ctl) + sizeof(unsigned long long) * (size_t)it,
                                     cudaMemcpyDeviceToHost, c->stream));
         CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-        if (c->ctlHost->jacobiDone) {
-            done = c->ctlHost->jacobiDone;
-            break;
+        done = c->ctlHost->jacobiDone;
+        for (int n = std::max(from, it - 2); n < it && !done; ++n) {
+            double change;
+            std::memcpy(&change, &c->ctlHost->res[n], sizeof(double));
+            if (change < tol) done = n + 1;
         }
-        double last;
-        unsigned long long b = c->ctlHost->res[it - 1];
-        std::memcpy(&last, &b, sizeof(double));
-        if (last < tol) {
-            done = it;
-            break;
-        }
+        if (done) break;
         batch = first && batch > 4 ? 4 : std::min(batch * 2, 32);
         first = false;
     }
     iters = done ? done : maxIter;
     c->jacPrevIters = iters;
-    result = (iters & 1) ? c->F.pB : c->F.pA;
+    if (pairs) {
+        // pair m wrote iterate 2 m + 2 and left its input, iterate 2 m
+        const int m = iters / 2;
+        if ((iters & 1) && iters < it) {
+            CUDA_TRY(c, cudaMemsetAsync(&c->ctl->jacobiDone, 0, sizeof(int), c->stream));
+            st = single(iters - 1, buf[m & 1], buf[(m & 1) ^ 1]);
+            if (st != SIFV_OK) return st;
+        }
+        result = buf[(m + (iters & 1)) & 1];
+    } else {
+        result = buf[iters & 1];
+    }
     mark(c, "jacobi");
     return SIFV_OK;
 }
@@ -1104,24 +1165,6 @@ int mg_alloc(sifv_ctx* c) {
     while (T.first + 1 < T.n && mg[T.first].n > kMgTail) ++T.first;
     for (int l = 0; l < T.n; ++l) T.l[l] = mg[l];
     c->mg = mg;
-    return SIFV_OK;
-}
-
-// A kernel of a chain whose every kernel waits for the one before it
-// (grid_dep_wait): set up while that one still runs.
-template <typename... KArgs, typename... Args>
-int launch_chained(sifv_ctx* c, void (*kernel)(KArgs...), unsigned grid, unsigned threads, Args... args) {
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3(grid);
-    lc.blockDim = dim3(threads);
-    lc.stream = c->stream;
-    lc.attrs = at;
-    lc.numAttrs = 1;
-    CUDA_TRY(c, cudaLaunchKernelEx(&lc, kernel, KArgs(args)...));
-    c->launches++;
     return SIFV_OK;
 }
 
@@ -2370,7 +2413,7 @@ int sifv_pressure_solve(sifv_ctx_t* c, const double* rho, const double* rhoc2, c
         CUDA_TRY(c, cudaMemcpyAsync(dP, res, bytes, cudaMemcpyDeviceToDevice, c->stream));
     else
         k_jacobi_finish<<<blocks((long long)c->nint, kCellThreads), kCellThreads, 0, c->stream>>>(
-            c->P, c->F.pA, c->F.pB, dP, c->ctl, maxIter);
+            c->P, res, res, dP, c->ctl, maxIter);
     LAUNCH_CHECK(c);
     if (!onDevice) CUDA_TRY(c, cudaMemcpyAsync(pressure, dP, bytes, cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));

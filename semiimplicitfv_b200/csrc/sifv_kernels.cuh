@@ -982,6 +982,17 @@ __device__ __forceinline__ double jacobi_pre_cell(const Params& P, const double*
     return jacobi_pre_update(P, coef, nc, rhs, pin, pout, jacobi_nb(P, i, j, k));
 }
 
+// The check before iteration it: true when an earlier change was
+// below tol (then jacobiDone is the number of iterations taken).
+__device__ __forceinline__ bool jacobi_stop(Ctl* ctl, int it, double tol) {
+    if (ctl->jacobiDone) return true;
+    int done = 0;
+    if (it >= 1 && bits2d(ctl->res[it - 1]) < tol) done = it;
+    if (it >= 2 && bits2d(ctl->res[it - 2]) < tol) done = it - 1;   // inside a pair (k_jacobi3_pair)
+    if (done && threadIdx.x == 0) ctl->jacobiDone = done;
+    return done != 0;
+}
+
 // Grid-stride Jacobi iteration (a grid of a few blocks per SM, two cells in
 // flight per thread): the convergence check, the block reduction and the
 // residual atomic run once per block instead of once per 256 cells.  A NaN
@@ -989,11 +1000,9 @@ __device__ __forceinline__ double jacobi_pre_cell(const Params& P, const double*
 __global__ void __launch_bounds__(256) k_jacobi_pre(Params P, const double* __restrict__ coef, size_t nc,
                                                     const double* __restrict__ rhs, const double* __restrict__ pin,
                                                     double* __restrict__ pout, Ctl* ctl, int it, double tol) {
-    if (ctl->jacobiDone) return;
-    if (it > 0 && bits2d(ctl->res[it - 1]) < tol) {
-        if (threadIdx.x == 0) ctl->jacobiDone = it;
-        return;
-    }
+    grid_dep_launch();
+    grid_dep_wait();
+    if (jacobi_stop(ctl, it, tol)) return;
     const long long tot = (long long)P.nx * P.ny * P.nz;
     const long long stride = (long long)gridDim.x * blockDim.x;
     double res = 0.0;
@@ -1101,11 +1110,9 @@ __global__ void __launch_bounds__(256) k_jacobi_face(Params P, const double* __r
                                                      const double* __restrict__ rhoc2,
                                                      const double* __restrict__ rhs, const double* __restrict__ pin,
                                                      double* __restrict__ pout, Ctl* ctl, int it, double tol) {
-    if (ctl->jacobiDone) return;
-    if (it > 0 && bits2d(ctl->res[it - 1]) < tol) {
-        if (threadIdx.x == 0) ctl->jacobiDone = it;
-        return;
-    }
+    grid_dep_launch();
+    grid_dep_wait();
+    if (jacobi_stop(ctl, it, tol)) return;
     const double dt = ctl->dt;
     const double dt2 = dt * dt;
     const long long tot = (long long)P.nx * P.ny * P.nz;
@@ -1194,11 +1201,9 @@ __global__ void __launch_bounds__(256, 3) k_jacobi3(Params P, const double* __re
                                                  const double* __restrict__ rhoc2, const double* __restrict__ rhs,
                                                  const double* __restrict__ pin, double* __restrict__ pout, Ctl* ctl,
                                                  int it, double tol) {
-    if (ctl->jacobiDone) return;
-    if (it > 0 && bits2d(ctl->res[it - 1]) < tol) {
-        if (threadIdx.x == 0) ctl->jacobiDone = it;
-        return;
-    }
+    grid_dep_launch();
+    grid_dep_wait();
+    if (jacobi_stop(ctl, it, tol)) return;
     const int i = (int)blockIdx.x * 32 + (int)(threadIdx.x & 31);
     const int j = (int)blockIdx.y * 8 + (int)(threadIdx.x >> 5);
     const int k0 = (int)blockIdx.z * kJacZ;
@@ -1222,6 +1227,252 @@ __global__ void __launch_bounds__(256, 3) k_jacobi3(Params P, const double* __re
         }
     }
     block_max_to(res, &ctl->res[it]);
+}
+
+// 8-byte asynchronous global -> shared copy (cp.async, L1-allocating) and
+// the wait for all of this thread's outstanding copies.
+__device__ __forceinline__ void cp_async8(double* smemDst, const double* gmemSrc) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(smemDst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(gmemSrc) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+template <int OFFSET>   // the same to a shared-memory address plus OFFSET bytes
+__device__ __forceinline__ void cp_async8_at(unsigned smemDst, const double* gmemSrc) {
+    asm volatile("cp.async.ca.shared.global [%0 + %1], [%2], 8;\n" ::"r"(smemDst), "n"(OFFSET), "l"(gmemSrc) : "memory");
+}
+__device__ __forceinline__ void cp_async16(void* smemDst, const void* gmemSrc) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(smemDst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gmemSrc) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+// Two 3D Jacobi iterations, it and it + 1, in one pass over memory.  An
+// iteration alone moves 56 bytes per cell for some 50 operations; two of them
+// share the coefficients, the right-hand side and the denominator with its
+// reciprocal, and the iterate between them stays on the chip.
+//
+// A block owns kJac2Y rows of 32 columns and walks a segment of planes.  Warp b
+// of the first kJac2Y + 2 takes row b - 1 (the rows outside are the first
+// iteration's halo), one more warp the columns to the left and the right.
+// Each thread copies the operands of its column two planes ahead into a ring
+// in shared memory (cp.async: no registers, and the latency of a plane's
+// worth of DRAM is hidden with one block per SM); the neighbours' values are
+// read there, or, past the block's halo, from a copy of the thread's own.  Per
+// plane every thread forms iterate it + 1 of its column; past the one barrier
+// the owners form iterate it + 2 of the plane below, with the operands of the
+// step before still in registers.  A halo position outside the mesh is
+// computed as the cell that the ghost map takes it from, and the quotients are
+// the correctly rounded ones (div_markstein, or the plain division out of its
+// range), so every iterate is the one that two launches give, bit for bit.
+// Both changes are reduced.  If iterate it + 1 is the converged one, the input
+// is still there and one single iteration gives it again.
+//
+// Per iteration, k_jacobi3 against this: 256^3 214 -> 166 us, 200 x 180 x 160
+// 88 -> 72, 128^3 43 -> 27, 64^3 27.5 -> 7.3 (whose walks of 32 planes were
+// the time).  Issue slots are 63 % busy; fetched with plain loads a plane
+// ahead, the same pair took 232 at 256^3.
+constexpr int kJac2Y = 16;
+constexpr int kJac2Threads = 32 * (kJac2Y + 3);
+constexpr int kJac2Row = 36;   // shared row of iterate it + 1: columns -1 .. 32
+constexpr int kJac2Ring = 3;
+template <bool FACE>
+__host__ __device__ constexpr int jac2_arrays() { return FACE ? 12 : 14; }
+template <bool FACE>
+constexpr size_t jac2_smem() {
+    return sizeof(double) * ((size_t)kJac2Ring * jac2_arrays<FACE>() * kJac2Threads + 3 * (kJac2Y + 2) * kJac2Row);
+}
+
+// The operands of one column's cell for a pair of iterations.
+template <bool FACE>
+struct JacPair {
+    double rh, co, dn, y, c0, c1, c2, c3, c4, c5;   // y = RN(1 / dn)
+    bool fast;                                      // dn is in div_markstein's range
+    __device__ __forceinline__ double update(double xm, double xp, double ym, double yp, double zm, double zp) const {
+        double od = 0.0;
+        od += c0 * xm + c1 * xp;
+        od += c2 * ym + c3 * yp;
+        od += c4 * zm + c5 * zp;
+        const double n = rh + co * od;
+        double q = div_markstein(n, dn, y);
+        if (!(fast && rn_fast_operand(n))) q = n / dn;
+        return q;
+    }
+    // the denominator (jacobi_face_update) and its reciprocal; co is rho c^2 on entry
+    __device__ __forceinline__ void prepare(double dt2) {
+        if (FACE) {
+            co = co * dt2;
+            double diag = 0.0;
+            diag += c0 + c1;
+            diag += c2 + c3;
+            diag += c4 + c5;
+            dn = 1.0 + co * diag;
+        }
+        y = rcp_rn(dn, rcp_near(dn));
+        fast = rn_fast_recip(y) && __double2loint(dn) != -1;
+    }
+};
+
+template <bool FACE>
+__global__ void __launch_bounds__(kJac2Threads, 1) k_jacobi3_pair(
+    Params P, const double* __restrict__ coef, size_t nc, const double* __restrict__ rhoc2,
+    const double* __restrict__ rhs, const double* __restrict__ pin, double* __restrict__ pout, Ctl* ctl, int it,
+    double tol, int segPlanes) {
+    constexpr int TY = kJac2Y, NT = kJac2Threads, NA = jac2_arrays<FACE>();
+    // arrays of a ring slot: rhs, rho c^2 (or its dt^2 multiple), c0, c2, c5, pin, pin of the four neighbours where no
+    // thread of the block holds it, then c1, c3 likewise (FACE) or c1, c3, c4, denominator
+    enum { RH, CO, C0, C2, C5, PZ, XM, XP, YM, YP, C1, C3, C4, DN };
+    extern __shared__ __align__(16) double jac2Smem[];
+    double* const ring = jac2Smem;
+    double* const sP = ring + kJac2Ring * NA * NT;   // iterate it + 1, three planes
+    grid_dep_launch();
+    grid_dep_wait();
+    if (jacobi_stop(ctl, it, tol)) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int i0 = (int)blockIdx.x * 32, j0 = (int)blockIdx.y * TY;
+    const int z0 = (int)blockIdx.z * segPlanes, z1 = min(z0 + segPlanes, P.nz);
+    const int lx = min(32, P.nx - i0), ly = min(TY, P.ny - j0);
+    auto srcX = [&](int i) { return scalar_src(i, P.nx, P.bc[0], P.bc[1]); };
+    auto srcY = [&](int j) { return scalar_src(j, P.ny, P.bc[2], P.bc[3]); };
+    auto srcZ = [&](int k) { return scalar_src(k, P.nz, P.bc[4], P.bc[5]); };
+    // the thread that holds position (a, b), -1 for none
+    auto holder = [&](int a, int b) {
+        if (a > lx || b > ly || a < -1 || b < -1) return -1;
+        if (a >= 0 && a < 32) return 32 * (b + 1) + a;
+        return (b >= 0 && b < ly) ? 32 * (TY + 2) + (a < 0 ? 0 : TY) + b : -1;
+    };
+    int a = lane, b = warp - 1;   // the thread's column
+    if (warp == TY + 2) {
+        a = (lane & TY) ? 32 : -1;
+        b = lane & (TY - 1);
+    }
+    const bool on = holder(a, b) == tid;
+    const bool own = on && warp < TY + 2 && a < lx && b >= 0 && b < ly;
+    const int pos = (a + 1) + kJac2Row * (b + 1);
+    const double dt = ctl->dt, dt2 = dt * dt;
+    const int si = on ? srcX(i0 + a) : 0, sj = on ? srcY(j0 + b) : 0;
+    const unsigned sy = (unsigned)P.nxT, sz = sy * (unsigned)P.nyT, col = (unsigned)cidx(P, si, sj, 0);
+    // where the neighbours' values are: another thread's slot, or the thread's own copies
+    int qXM = XM * NT + tid, qXP = XP * NT + tid, qYM = YM * NT + tid, qYP = YP * NT + tid, qC1 = C1 * NT + tid,
+        qC3 = C3 * NT + tid;
+    int oXM = 0, oXP = 0, oYM = 0, oYP = 0;   // else the distance to load them from
+    {
+        auto place = [&](int& q, int& o, int h, bool same, int array, int distance) {
+            if (h >= 0 && same) q = array * NT + h; else o = distance;
+        };
+        place(qXM, oXM, holder(a - 1, b), srcX(i0 + a - 1) == srcX(si - 1), PZ, srcX(si - 1) - si);
+        place(qXP, oXP, holder(a + 1, b), srcX(i0 + a + 1) == srcX(si + 1), PZ, srcX(si + 1) - si);
+        place(qYM, oYM, holder(a, b - 1), srcY(j0 + b - 1) == srcY(sj - 1), PZ, (srcY(sj - 1) - sj) * (int)sy);
+        place(qYP, oYP, holder(a, b + 1), srcY(j0 + b + 1) == srcY(sj + 1), PZ, (srcY(sj + 1) - sj) * (int)sy);
+        if (FACE) {   // the high faces: the next cell's low ones
+            int o = 0;
+            place(qC1, o, holder(a + 1, b), srcX(i0 + a + 1) == si + 1, C0, 0);
+            place(qC3, o, holder(a, b + 1), srcY(j0 + b + 1) == sj + 1, C2, 0);
+        }
+    }
+    const bool dXM = qXM == XM * NT + tid, dXP = qXP == XP * NT + tid, dYM = qYM == YM * NT + tid,
+               dYP = qYP == YP * NT + tid, dC1 = qC1 == C1 * NT + tid, dC3 = qC3 == C3 * NT + tid;
+    const double* const coefY = coef + nc * (FACE ? 1 : 2);
+    const double* const coefZ = coef + nc * (FACE ? 2 : 4);
+    const bool extra = on && (dXM || dXP || dYM || dYP || (FACE && (dC1 || dC3)));   // rows and columns of the halo only
+    const unsigned ringAt = (unsigned)__cvta_generic_to_shared(ring) + 8u * (unsigned)tid;
+    constexpr int kSlot = NA * NT;
+    auto fetch = [&](bool wanted, int k, int slot) {   // the operands of source plane k into a ring slot
+        if (on && wanted) {
+            const unsigned c = col + sz * (unsigned)k;
+            const unsigned s = ringAt + 8u * (unsigned)slot;
+            cp_async8_at<8 * RH * NT>(s, rhs + c);
+            cp_async8_at<8 * PZ * NT>(s, pin + c);
+            cp_async8_at<8 * C0 * NT>(s, coef + c);
+            cp_async8_at<8 * C2 * NT>(s, coefY + c);
+            if (FACE) {
+                cp_async8_at<8 * CO * NT>(s, rhoc2 + c);
+                cp_async8_at<8 * C5 * NT>(s, coefZ + (c + sz));
+            } else {
+                cp_async8_at<8 * C1 * NT>(s, coef + nc + c);
+                cp_async8_at<8 * C3 * NT>(s, coefY + nc + c);
+                cp_async8_at<8 * C4 * NT>(s, coefZ + c);
+                cp_async8_at<8 * C5 * NT>(s, coefZ + nc + c);
+                cp_async8_at<8 * CO * NT>(s, coef + 6 * nc + c);
+                cp_async8_at<8 * DN * NT>(s, coef + 7 * nc + c);
+            }
+            if (extra) {
+                if (dXM) cp_async8_at<8 * XM * NT>(s, pin + (c + oXM));
+                if (dXP) cp_async8_at<8 * XP * NT>(s, pin + (c + oXP));
+                if (dYM) cp_async8_at<8 * YM * NT>(s, pin + (c + oYM));
+                if (dYP) cp_async8_at<8 * YP * NT>(s, pin + (c + oYP));
+                if (FACE && dC1) cp_async8_at<8 * C1 * NT>(s, coef + (c + 1));
+                if (FACE && dC3) cp_async8_at<8 * C3 * NT>(s, coefY + (c + sy));
+            }
+        }
+        cp_async_commit();
+    };
+    double res1 = 0.0, res2 = 0.0, below = 0.0, centre = 0.0;
+    JacPair<FACE> keep = {};
+    int kA = srcZ(z0 - 1), kB = srcZ(z0);   // source planes of positions kk, kk + 1
+    int rA = 0, rB = kSlot, rC = 2 * kSlot;                                  // their ring slots, and the next one's
+    int pA = 0, pB = (TY + 2) * kJac2Row, pC = 2 * (TY + 2) * kJac2Row;      // planes kk, kk - 1, kk - 2 of iterate it + 1
+    fetch(true, kA, rA);
+    fetch(true, kB, rB);
+    cp_async_wait_group<1>();
+    __syncthreads();
+    bool follows = false;             // position kk is the plane above position kk - 1's
+    double zm = 0.0, c5Last = 0.0;    // pin and the high z face of that plane
+#pragma unroll 1   // unrolled by 2 or 6: 20 % and 29 % slower at 256^3
+    for (int kk = z0 - 1; kk <= z1; ++kk) {
+        const int kC = srcZ(kk + 2);
+        fetch(kk + 2 <= z1, kC, rC);
+        double pn = 0.0, pc = 0.0;
+        JacPair<FACE> cur = {};
+        cp_async_wait_group<1>();   // the thread's share of position kk + 1
+        const bool next = kB == kA + 1 && kk < z1;
+        if (on) {
+            const double* const s = ring + rA;
+            cur.rh = s[RH * NT + tid];
+            cur.co = s[CO * NT + tid];
+            cur.c0 = s[C0 * NT + tid];
+            cur.c1 = s[qC1];
+            cur.c2 = s[C2 * NT + tid];
+            cur.c3 = s[qC3];
+            cur.c5 = s[C5 * NT + tid];
+            cur.c4 = FACE ? c5Last : s[C4 * NT + tid];
+            if (!FACE) cur.dn = s[DN * NT + tid];
+            pc = s[PZ * NT + tid];
+            double zp = ring[rB + PZ * NT + tid];
+            if (!next) zp = pin[col + sz * (unsigned)srcZ(kA + 1)];   // the ghost map's jump, or the last position
+            if (!follows) {
+                zm = pin[col + sz * (unsigned)srcZ(kA - 1)];
+                if (FACE) cur.c4 = coefZ[col + sz * (unsigned)kA];
+            }
+            cur.prepare(dt2);
+            pn = cur.update(s[qXM], s[qXP], s[qYM], s[qYP], zm, zp);
+            sP[pA + pos] = pn;
+            if (own && kk >= z0 && kk < z1) res1 = smax(res1, fabs(pn - pc));
+        }
+        __syncthreads();
+        if (own && kk > z0) {
+            const double* const q = sP + pB + pos;
+            const double p2 = keep.update(q[-1], q[1], q[-kJac2Row], q[kJac2Row], below, pn);
+            pout[col + sz * (unsigned)(kk - 1)] = p2;
+            res2 = smax(res2, fabs(p2 - centre));
+        }
+        below = centre;
+        centre = pn;
+        keep = cur;
+        zm = pc;
+        c5Last = cur.c5;
+        follows = next;
+        kA = kB;
+        kB = kC;
+        const int r = rA, p = pC;
+        rA = rB; rB = rC; rC = r;
+        pC = pB; pB = pA; pA = p;
+    }
+    cp_async_wait_group<0>();
+    block_max_to(res1, &ctl->res[it]);
+    __syncthreads();
+    block_max_to(res2, &ctl->res[it + 1]);
 }
 
 // Copy the converged Jacobi iterate (in pA or pB by parity) to dst.
@@ -1551,14 +1802,6 @@ __global__ void k_igr_sweep_1d(Params P, Fields F) {
     for (int i = 0; i < P.nx; ++i) igr_cell(P, F, i, 0, 0);
 }
 
-// 8-byte asynchronous global -> shared copy (cp.async, L1-allocating) and
-// the wait for all of this thread's outstanding copies.
-__device__ __forceinline__ void cp_async8(double* smemDst, const double* gmemSrc) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(smemDst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(gmemSrc) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-
 // Sweeps of one IGR solve overlapped in one launch sequence (k_igr_tile,
 // k_igr_tile_rec): the tile plane of each active sweep, and whether the
 // boundary tiles refresh the scalar ghost layer themselves.
@@ -1814,13 +2057,6 @@ __global__ void __launch_bounds__(256) k_igr_records(Params P, Fields F, double*
         atomicOr(slowRecs, 1);
 }
 
-__device__ __forceinline__ void cp_async16(void* smemDst, const void* gmemSrc) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(smemDst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gmemSrc) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 // The tiled wavefront of k_igr_tile<16, 16, 16> (same tile planes, same cell
 // planes inside a tile, igr_cell's arithmetic in igr_cell's order) with
