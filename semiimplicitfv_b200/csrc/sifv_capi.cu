@@ -1474,9 +1474,17 @@ void flush_advance(sifv_ctx* c) {
 // exchange, immersed bodies, the adjoint's and tangent's hooks) and no
 // capillary stress is added.  One-stage schemes would need their output
 // copied back over their input and keep the separate kernels.
+//
+// The fast and mixed modes take it too on 1D meshes up to kStageFastCells:
+// the six kernels and the dt pass of their step are launch latency there
+// (95 / 107 us per step mixed / FP64 at 20000 cells, where this takes 27; 109
+// / 118 at 262145, against 113), and beyond it their cheaper arithmetic wins
+// (121 / 136 against 161 us at 400000).
+constexpr int kStageFastCells = 240000;
 bool fused_stage(const sifv_ctx* c) {
     const Params& P = c->P;
-    return c->cfg.precision == SIFV_PREC_FP64 && !c->cfg.semiImplicit && !c->cfg.useIGR && P.dim <= 2 && c->W == 5 &&
+    const bool mode = c->cfg.precision == SIFV_PREC_FP64 || (c->sweep && P.dim == 1 && P.nx <= kStageFastCells);
+    return mode && !c->cfg.semiImplicit && !c->cfg.useIGR && P.dim <= 2 && c->W == 5 &&
            c->nphT <= 2 && c->cfg.RKOrder > 1 && !P.cap && !c->ib.count && !c->F.solid && !c->exchangeFaces &&
            !c->stageHook && P.ngx <= kStageMaxGhost && P.ny <= 8 * 65535;
 }
@@ -1752,7 +1760,7 @@ int enqueue_step(sifv_ctx* c, int step, double time, double targetDt, int useEnd
         c->dtReady = fold;
         return SIFV_OK;
     }
-    if (c->sweep) {
+    if (c->sweep && !fused_stage(c)) {
         SweepArgs A{};
         A.P = c->P;
         A.F = c->F;
@@ -2106,7 +2114,7 @@ int sifv_create(const sifv_config_t* cfg, const sifv_mesh_t* mesh, int device, s
     F.dx = g[0]; F.dy = g[1]; F.dz = g[2]; F.adx2 = g[3]; F.ady2 = g[4]; F.adz2 = g[5];
     if (cfg->precision != SIFV_PREC_FP64 && !cfg->semiImplicit) {
         c->sweep = true;
-        if (dim == 1) {
+        if (dim == 1 && !fused_stage(c)) {
             c->rhoP = dalloc(c, n, st);
             c->rhsBuf[0] = dalloc(c, n, st);
             c->rhsBuf[1] = dalloc(c, n, st);
