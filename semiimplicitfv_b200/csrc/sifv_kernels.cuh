@@ -10,8 +10,9 @@
 //   k_assemble     per cell: flux divergence in the reference's accumulation
 //                  order, sources, and the SSP-RK update (or the
 //                  semi-implicit star update), fused
-// The semi-implicit stage adds k_bc_prim, k_pressure_setup, the Jacobi
-// iterations (k_jacobi) and k_correction.  IGR runs k_igr_setup and, per
+// (in 1D and 2D most explicit configurations run these as one kernel,
+// sifv_stage.cuh).  The semi-implicit stage adds k_bc_prim, k_pressure_setup,
+// the Jacobi iterations (k_jacobi3_pair in 3D) and k_correction.  IGR runs k_igr_setup and, per
 // sweep, one k_igr_tile launch per tile plane of the lexicographic
 // Gauss-Seidel sweep (the dependency order of src/IGR.cpp:110-156).
 #pragma once
