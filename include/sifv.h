@@ -82,7 +82,7 @@ extern "C" {
 /* arithmetic of the reconstruction/flux bulk */
 #define SIFV_PREC_FP64      0   /* FP64 in the reference's operation order: bit-identical results */
 #define SIFV_PREC_MIXED     1   /* FP32 reconstruction/flux bulk; FP64 state, primitive recovery, divergence, RK update */
-#define SIFV_PREC_FP64_FAST 2   /* FP64, fused sweeps with reassociated arithmetic (FMA, shared WENO indicators) */
+#define SIFV_PREC_FP64_FAST 2   /* FP64, fused kernels with reassociated arithmetic (FMA, shared WENO indicators) */
 /* SIFV_PREC_MIXED and SIFV_PREC_FP64_FAST run the explicit single-phase
  * WENO5 step (any dim, any Riemann solver, no IGR, no body force); other
  * configurations are rejected by sifv_create with SIFV_ERR_UNSUPPORTED. */
