@@ -638,11 +638,13 @@ __global__ void __launch_bounds__(128) k_adj_cell(const __grid_constant__ AdjArg
 }
 
 // ---------------------------------------------------------------------------
-// Tangent (forward mode).
+// Tangent (forward mode).  A device-resident run queues steps past its end
+// time that the state kernels skip; so do these (A.skip).
 // ---------------------------------------------------------------------------
 // dW of every cell (ghosts: the source cell's dW with the velocity signs)
 template <int DIM>
 __global__ void __launch_bounds__(256) k_tan_prim(AdjArgs A) {
+    if (A.skip && *A.skip) return;
     const Params& P = A.P;
     const Fields& F = A.F;
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -678,6 +680,7 @@ __global__ void __launch_bounds__(256) k_tan_prim(AdjArgs A) {
 
 template <int DIR, int DIM>
 __global__ void __launch_bounds__(128) k_tan_face(AdjArgs A) {
+    if (A.skip && *A.skip) return;
     constexpr int NVN = NV<DIM>::n;
     const Params& P = A.P;
     const Fields& F = A.F;
@@ -725,6 +728,7 @@ __global__ void __launch_bounds__(128) k_tan_face(AdjArgs A) {
 
 template <int DIM>
 __global__ void __launch_bounds__(256) k_tan_update(AdjArgs A, int save) {
+    if (A.skip && *A.skip) return;
     constexpr int NVN = NV<DIM>::n;
     const Params& P = A.P;
     const Fields& F = A.F;

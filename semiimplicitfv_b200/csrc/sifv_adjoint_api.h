@@ -16,6 +16,7 @@ struct AdjArgs {
     double* gdir[3][5];  // dJ/dW per direction (all cells; ghost positions within three layers)
     double dt, a1, a2, a3;   // dt and c1/c4, c2/c4, c3/c4 of the stage
     const double* dtDev;     // non-null: dt is read from device memory (the step's CFL dt)
+    const int* skip;         // non-null: the tangent kernels of a skipped step (*skip != 0) do nothing
     int stage0;          // stage 0 of a step: lam += acc0, acc0 = 0
     unsigned adjTiles;   // blocks along a grid line of the reverse kernel (set by the launcher)
     int fp32;            // local Jacobians of the reverse sweep in FP32

@@ -2938,6 +2938,7 @@ int sifv_tangent_forward(sifv_ctx_t* c, int step0, double time0, double tEnd, in
         AdjArgs A = adj_args(c);
         set_stage_coef(A, RK, s);
         A.dtDev = &c->ctl->dt;
+        A.skip = &c->ctl->skip;   // run_forward queues steps past tEnd
         if (phase == 1) return tangent_faces(A, c->stream);
         return tangent_update(A, (s == 0 && RK > 1) ? 1 : 0, c->stream);
     };
