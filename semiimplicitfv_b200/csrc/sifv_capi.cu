@@ -2639,6 +2639,14 @@ struct HookGuard {
     }
 };
 
+// Clears the control block's skip flag when a forward run returns: its last
+// batch may have been queued past the end time, and the kernels of later
+// calls would skip their work too.
+struct SkipGuard {
+    sifv_ctx* c;
+    ~SkipGuard() { cudaMemsetAsync(&c->ctl->skip, 0, sizeof(int), c->stream); }
+};
+
 // Forward steps from the current state, either with a given time-step
 // sequence or with the CFL dt and targetDt = tEnd - t; optionally records
 // the sequence and a checkpoint every `every` steps.  The steps between two
@@ -2658,6 +2666,7 @@ int run_forward(sifv_ctx* c, int step0, double time0, double tEnd, int maxSteps,
     h.time = time0;
     h.tEnd = sched ? INFINITY : tEnd;
     CUDA_TRY(c, cudaMemcpyAsync(c->ctl, &h, offsetof(Ctl, res), cudaMemcpyHostToDevice, c->stream));
+    SkipGuard skip{c};
     for (;;) {
         int left = sched ? nSched - q : (maxSteps > 0) ? maxSteps - q : batchMax;
         if (left <= 0 || (!sched && !(t < tEnd))) break;
@@ -2892,6 +2901,7 @@ int sifv_adjoint_backward(sifv_ctx_t* c, double* deviceMs) {
     // the context's state is the end of the forward run again
     st = load_checkpoint(c, (size_t)nSeg);
     if (st != SIFV_OK) return st;
+    CUDA_TRY(c, cudaMemsetAsync(&c->ctl->skip, 0, sizeof(int), c->stream));   // a sifv_advance in between may have set it
     launch_prim_bc(c);
     for (int q = 0; q < nv; ++q)
         if (zero_ghosts(c->P, c->lam[q], c->stream) != 0) return fail(c, SIFV_ERR_CUDA, "launch failed");

@@ -64,3 +64,25 @@ def test_tangent_to_an_end_time_takes_the_recorded_steps(name, rk):
     for f in v:
         for a, b in zip(free[f], fixed[f]):
             assert np.array_equal(a, b), f
+
+
+@pytest.mark.parametrize("between", ["overwritten", "advanced"])
+@pytest.mark.parametrize("name", ["constant", "growing", "growing_2d"])
+def test_backward_restores_the_end_state_whatever_came_between(name, between):
+    make, t_end, _ = CASES[name]
+    case = make()
+    dim = case[0].dim
+    ctx = backends.make(backends.cuda(), case)
+    t, n = ctx.adjoint_forward(0, 0.0, t_end, 0, 64)
+    fids = cons_fids(dim) + [abi.F_VELU, abi.F_PRES] + ([abi.F_VELV] if dim == 2 else [])
+    end = {f: ctx.get_field(f) for f in fids}
+    if between == "overwritten":
+        for f in fids:
+            ctx.set_field(f, np.full(ctx.shape, 7.0))
+    else:   # to an end time, with steps to spare
+        assert ctx.advance(n, t, t + 2.5 * t / n, 6)[1] < 6
+    for f in cons_fids(dim):
+        ctx.adjoint_set_seed(f, np.ones(ctx.shape))
+    ctx.adjoint_backward()
+    for f in fids:
+        assert np.array_equal(ctx.get_field(f), end[f]), f
