@@ -1704,7 +1704,7 @@ int enqueue_step(sifv_ctx* c, int step, double time, double targetDt, int useEnd
                 return fail(c, SIFV_ERR_CUDA, "tile launch failed");
             }
         }
-        if (RK == 1 && state_copy(c->ctl, c->tileB, U, 4, c->ncells, c->stream, c->launches) != 0)
+        if (RK == 1 && tile2d_copy(c->ctl, c->tileB, U, c->ncells, c->stream, c->launches) != 0)
             return fail(c, SIFV_ERR_CUDA, "copy launch failed");
         launch_bc_prim(c);
         LAUNCH_CHECK(c);
@@ -1753,7 +1753,7 @@ int enqueue_step(sifv_ctx* c, int step, double time, double targetDt, int useEnd
                 return fail(c, SIFV_ERR_CUDA, "tile launch failed");
             }
         }
-        if (RK == 1 && state_copy(c->ctl, c->tileB, U, 5, c->ncells, c->stream, c->launches) != 0)
+        if (RK == 1 && tile3d_copy(P, c->ctl, c->tileB, U, c->stream, c->launches) != 0)
             return fail(c, SIFV_ERR_CUDA, "copy launch failed");
         launch_bc_prim(c);
         LAUNCH_CHECK(c);

@@ -106,15 +106,14 @@ int tile2d_stage(const TileArgs& A, cudaStream_t s, bool mixed, int& launches, L
     return st;
 }
 
-int state_copy(const Ctl* ctl, const double* const* in, double* const* out, int count, size_t n, cudaStream_t s,
-               int& launches) {
-    CopyN C{};
-    C.count = count;
-    for (int q = 0; q < count; ++q) {
+int tile2d_copy(const Ctl* ctl, const double* const in[4], double* const out[4], size_t n, cudaStream_t s,
+                int& launches) {
+    Copy4 C;
+    for (int q = 0; q < 4; ++q) {
         C.src[q] = in[q];
         C.dst[q] = out[q];
     }
-    k_copy_state<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(ctl, C, n);
+    k_copy4<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(ctl, C, n);
     ++launches;
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
@@ -179,6 +178,19 @@ int tile3d_stage(const Tile3Args& A, cudaStream_t s, bool mixed, int& launches, 
     ++launches;
     if (mark) mark(user, "tile3d");
     return st;
+}
+
+int tile3d_copy(const Params& P, const Ctl* ctl, const double* const in[5], double* const out[5], cudaStream_t s,
+                int& launches) {
+    Copy5 C;
+    for (int q = 0; q < 5; ++q) {
+        C.src[q] = in[q];
+        C.dst[q] = out[q];
+    }
+    const long long n = (long long)P.nx * P.ny * P.nz;
+    k_copy_interior<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(P, ctl, C);
+    ++launches;
+    return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
 namespace {

@@ -629,18 +629,16 @@ inline size_t march_mixed_smem() { return 4 * (5 * 2 * 36 * sizeof(float2) + 2 *
 
 // Stage output copied over the state (RK1, whose only stage cannot update
 // in place).
-struct CopyN {
-    const double* src[5];
-    double* dst[5];
-    int count;
+struct Copy4 {
+    const double* src[4];
+    double* dst[4];
 };
-__global__ void k_copy_state(const Ctl* ctl, CopyN A, size_t n) {
+__global__ void k_copy4(const Ctl* ctl, Copy4 A, size_t n) {
     if (ctl->skip) return;
     size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
 #pragma unroll
-    for (int q = 0; q < 5; ++q)
-        if (q < A.count) A.dst[q][t] = A.src[q][t];
+    for (int q = 0; q < 4; ++q) A.dst[q][t] = A.src[q][t];
 }
 
 }  // namespace sifv

@@ -94,9 +94,11 @@ int tile2d_stage(const TileArgs& A, cudaStream_t s, bool mixed, int& launches, L
                  void* user = nullptr);
 int tile3d_stage(const Tile3Args& A, cudaStream_t s, bool mixed, int& launches, LaunchMark mark = nullptr,
                  void* user = nullptr);
-// out[q] = in[q], q < count, over n values, skipped when the step is (device-side loops).
-int state_copy(const Ctl* ctl, const double* const* in, double* const* out, int count, size_t n, cudaStream_t s,
-               int& launches);
+// out[q] = in[q] over n values (2D) or the interior cells (3D), skipped when the step is (device-side loops).
+int tile2d_copy(const Ctl* ctl, const double* const in[4], double* const out[4], size_t n, cudaStream_t s,
+                int& launches);
+int tile3d_copy(const Params& P, const Ctl* ctl, const double* const in[5], double* const out[5], cudaStream_t s,
+                int& launches);
 
 // End-of-step conservative -> primitive on interior cells.
 int sweep_finish_prim(const Params& P, const Fields& F, const Ctl* ctl, cudaStream_t s, int& launches);

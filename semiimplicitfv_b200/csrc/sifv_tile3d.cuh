@@ -285,4 +285,21 @@ __global__ void __launch_bounds__(Tile3::threads, 2) k_tile3d(const __grid_const
     if (A.last && A.dtNext) block_min_to(limit, &A.ctl->dtBits);
 }
 
+// The stage output's interior cells copied over the state's (RK1, whose only
+// stage cannot update in place).  The scratch has no ghost layers of its own:
+// those of the state's momenta and energy stay as the caller left them, as in
+// the schemes of more stages.
+struct Copy5 {
+    const double* src[5];
+    double* dst[5];
+};
+__global__ void __launch_bounds__(256) k_copy_interior(Params P, const Ctl* ctl, Copy5 A) {
+    if (ctl->skip) return;
+    int i, j, k;
+    if (!int_coords(P, (long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
+    const size_t c = cidx(P, i, j, k);
+#pragma unroll
+    for (int q = 0; q < 5; ++q) A.dst[q][c] = A.src[q][c];
+}
+
 }  // namespace sifv
