@@ -246,13 +246,20 @@ int validate(const sifv_config_t* c, std::string& msg) {
 
 // n zeroed doubles that live as long as the context, 256-byte aligned.  Small
 // arrays share chunks of up to eight (64 MB at most): a cudaMalloc costs a
-// few tenths of a millisecond, and a context holds 20 to 60 arrays.
+// few tenths of a millisecond, and a context holds 20 to 60 arrays.  A chunk
+// is a whole number of arrays, and where there is no room for one the array
+// is allocated alone.
 double* dalloc(sifv_ctx* c, size_t n, int& st) {
     const size_t need = (std::max<size_t>(n, 1) * sizeof(double) + 255) / 256 * 256;
     if (c->arenaLeft < need) {
-        const size_t chunk = std::max(need, std::min<size_t>(8 * need, (size_t)64 << 20));
+        size_t chunk = need * std::max<size_t>(1, std::min<size_t>(8, ((size_t)64 << 20) / need));
         void* p = nullptr;
         cudaError_t e = cudaMalloc(&p, chunk);
+        if (e == cudaErrorMemoryAllocation && chunk > need) {
+            cudaGetLastError();   // handled here
+            chunk = need;
+            e = cudaMalloc(&p, chunk);
+        }
         if (e != cudaSuccess) {
             st = fail(c, SIFV_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
             return nullptr;
