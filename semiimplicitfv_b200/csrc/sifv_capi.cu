@@ -2612,6 +2612,12 @@ void free_checkpoints(sifv_ctx* c) {
     c->adjReady = false;
 }
 
+// The checkpoints not in use back to the device.
+void trim_pool(sifv_ctx* c) {
+    for (double* p : c->adjPool) cudaFree(p);
+    c->adjPool.clear();
+}
+
 // copy of the conservative state appended to the checkpoint list
 int push_checkpoint(sifv_ctx* c) {
     if (c->adjPool.empty()) {
@@ -2754,19 +2760,15 @@ int sifv_adjoint_forward(sifv_ctx_t* c, int step0, double time0, double tEnd, in
     double t = 0.0;
     int n = 0;
     st = run_forward(c, step0, time0, tEnd, maxSteps, dtSchedule, nSchedule, checkpointEvery, true, t, n);
-    if (st != SIFV_OK) {
+    if (st == SIFV_OK) st = push_checkpoint(c);   // final state, restored after the reverse sweep
+    if (st != SIFV_OK) {   // nothing is kept for a run that failed
         free_checkpoints(c);
-        return st;
-    }
-    st = push_checkpoint(c);   // final state, restored after the reverse sweep
-    if (st != SIFV_OK) {
-        free_checkpoints(c);
+        trim_pool(c);
         return st;
     }
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     c->adjReady = true;
-    for (double* p : c->adjPool) cudaFree(p);   // no more is kept than this run used
-    c->adjPool.clear();
+    trim_pool(c);   // no more is kept than this run used
     if (timeOut) *timeOut = t;
     if (stepsOut) *stepsOut = n;
     return SIFV_OK;

@@ -2,6 +2,7 @@
 end time do nothing: not to the state, not to the tangent, and not to the calls that follow."""
 import numpy as np
 import pytest
+import torch
 
 import backends
 import cases
@@ -86,3 +87,17 @@ def test_backward_restores_the_end_state_whatever_came_between(name, between):
     ctx.adjoint_backward()
     for f in fids:
         assert np.array_equal(ctx.get_field(f), end[f]), f
+
+
+def test_failed_forward_keeps_no_checkpoints():
+    """A forward run that fails gives the memory of its checkpoints, and of the earlier run's, back."""
+    ctx = backends.make(backends.cuda(), cases.vortex2d(1000))
+    ctx.adjoint_forward(0, 0.0, 1.0, 8, 4)   # three checkpoints
+    free = torch.cuda.mem_get_info()[0]
+    u = ctx.get_field(abi.F_VELU)
+    u[0, 500, 500] = np.inf   # the first time step is 0
+    ctx.set_field(abi.F_VELU, u)
+    with pytest.raises(abi.AbiError) as e:
+        ctx.adjoint_forward(0, 0.0, 1.0, 8, 4)
+    assert e.value.status == abi.ERR_NAN
+    assert torch.cuda.mem_get_info()[0] - free >= 3 * 4 * 8 * ctx.ncells
