@@ -2268,6 +2268,7 @@ int sifv_set_field(sifv_ctx_t* c, int field, const double* src, int onDevice) {
     double* p = field_ptr(c, field);
     if (!p) return fail(c, SIFV_ERR_BAD_ARG, "field not allocated for this configuration");
     cudaSetDevice(c->device);
+    c->dtReady = false;   // a time step folded from the old state (a progress callback writes this one)
     CUDA_TRY(c, cudaMemcpyAsync(p, src, c->ncells * sizeof(double),
                                 onDevice ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
@@ -2453,6 +2454,7 @@ int sifv_igr_solve(sifv_ctx_t* c, int step) {
 
 int sifv_acoustic_dt(sifv_ctx_t* c, double cfl, double maxDt, double* dt) {
     cudaSetDevice(c->device);
+    c->dtReady = false;   // its accumulator is used here
     CUDA_TRY(c, cudaMemsetAsync(&c->ctl->skip, 0, sizeof(int), c->stream));
     k_dt_init<<<1, 1, 0, c->stream>>>(c->ctl, maxDt);
     Fields Fa = c->F;
@@ -2469,6 +2471,7 @@ int sifv_acoustic_dt(sifv_ctx_t* c, double cfl, double maxDt, double* dt) {
 
 int sifv_advective_dt(sifv_ctx_t* c, double cfl, double maxDt, double* dt) {
     cudaSetDevice(c->device);
+    c->dtReady = false;   // its accumulator is used here
     CUDA_TRY(c, cudaMemsetAsync(&c->ctl->skip, 0, sizeof(int), c->stream));
     k_dt_init<<<1, 1, 0, c->stream>>>(c->ctl, maxDt);
     k_dt_advective<<<blocks((long long)c->nint, kCellThreads), kCellThreads, 0, c->stream>>>(c->P, c->F, c->ctl, cfl);
@@ -3248,6 +3251,7 @@ int sifv_run_time_loop(sifv_ctx_t* c, const sifv_time_loop_t* prm, sifv_vtk_t* v
         const bool due = c->ctlHost->outputDue != 0;
         int ran = 0;
         while (ran < B && log[ran] >= 0.0) ++ran;
+        bool called = false;
         for (int q = 0; q < ran; ++q) {   // the host's copy of the device's time arithmetic
             time += log[q];
             step++;
@@ -3259,8 +3263,14 @@ int sifv_run_time_loop(sifv_ctx_t* c, const sifv_time_loop_t* prm, sifv_vtk_t* v
                 st = output(time);
                 if (st != SIFV_OK) return finish(st);
             }
-            if (progress && (step % printEvery == 0 || step == 1)) progress(user, step, time, log[q]);
+            if (progress && (step % printEvery == 0 || step == 1)) {
+                progress(user, step, time, log[q]);
+                called = true;
+            }
         }
+        // the callback may have written the state through its device pointers; the 2D fast and mixed stages have always
+        // gone on with the limits they folded, which differ from the reduction's in the last bits
+        if (called && !(c->sweep && c->P.dim == 2)) c->dtReady = false;
         if (time != c->ctlHost->time) return finish(fail(c, SIFV_ERR_CUDA, "device and host time disagree"));
         if (due) {
             k_loop_resume<<<1, 1, 0, c->stream>>>(c->ctl);
