@@ -1,6 +1,4 @@
 // sifv_adjoint.cu -- launchers of the discrete adjoint and tangent kernels.
-#include <algorithm>
-
 #include "sifv_adjoint.cuh"
 
 namespace sifv {
@@ -19,17 +17,20 @@ int adj_dirs(const AdjArgs& A, cudaStream_t s) {
     if (cudaFuncSetAttribute(k_adj_dir<DIM, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return -1;
     const Params& P = A.P;
+    // every direction its own blocks, one after the other (a grid of the largest count in each direction is
+    // millions of empty blocks on an elongated mesh: 20000 x 4, gradient of 6 steps, 166 ms against 4.5)
     const long long n[3] = {P.nx, P.ny, P.nz};
-    long long tiles = 0, lines = 0;
-    for (int d = 0; d < DIM; ++d) {
-        tiles = std::max(tiles, (n[d] + 6 + kAdjOut - 1) / kAdjOut);
-        lines = std::max(lines, n[0] * n[1] * n[2] / n[d]);
-    }
-    const long long groups = (lines + kAdjLines - 1) / kAdjLines;
-    if (tiles * groups > 0x7fffffffLL) return -1;
     AdjArgs B = A;
-    B.adjTiles = (unsigned)tiles;
-    k_adj_dir<DIM, S><<<dim3((unsigned)(tiles * groups), DIM), kAdjLines * kAdjLen, smem, s>>>(B);
+    long long total = 0;
+    for (int d = 0; d < 3; ++d) {
+        B.adjFirst[d] = (unsigned)total;
+        if (d >= DIM) continue;
+        const long long tiles = (n[d] + 6 + kAdjOut - 1) / kAdjOut, lines = n[0] * n[1] * n[2] / n[d];
+        B.adjTiles[d] = (unsigned)tiles;
+        total += tiles * ((lines + kAdjLines - 1) / kAdjLines);
+        if (total > 0x7fffffffLL) return -1;
+    }
+    k_adj_dir<DIM, S><<<(unsigned)total, kAdjLines * kAdjLen, smem, s>>>(B);
     return 0;
 }
 

@@ -411,8 +411,8 @@ __device__ __forceinline__ void adj_dir(const AdjArgs& A, unsigned char* smem) {
     constexpr int NVN = NV<DIM>::n, LS = kAdjLines * kAdjStride;
     const Params& P = A.P;
     const int n = (D == 0) ? P.nx : (D == 1) ? P.ny : P.nz;
-    const int p0 = -3 + (int)(blockIdx.x % A.adjTiles) * kAdjOut;
-    if (p0 >= n + 3) return;
+    const unsigned block = blockIdx.x - A.adjFirst[D];
+    const int p0 = -3 + (int)(block % A.adjTiles[D]) * kAdjOut;
     double* const sSh = reinterpret_cast<double*>(smem);       // two buffers of five shares per cell
     S* const sW = reinterpret_cast<S*>(sSh + 2 * 5 * LS);      // primitives at p0 - 5 + index
     S* const sHi = sW + NVN * LS;                              // face values of cell p0 - 3 + index, then
@@ -422,7 +422,7 @@ __device__ __forceinline__ void adj_dir(const AdjArgs& A, unsigned char* smem) {
     const long long nLines = (long long)nt0 * ((D == 2) ? P.ny : P.nz);
     const int l = (D == 0) ? (int)threadIdx.x / kAdjLen : (int)threadIdx.x % kAdjLines;
     const int a = (D == 0) ? (int)threadIdx.x % kAdjLen : (int)threadIdx.x / kAdjLines;
-    const long long line = (long long)(blockIdx.x / A.adjTiles) * kAdjLines + l;
+    const long long line = (long long)(block / A.adjTiles[D]) * kAdjLines + l;
     const bool on = line < nLines;
     const int q0 = on ? (int)(line % nt0) : 0, q1 = on ? (int)(line / nt0) : 0;
     auto cell = [&](int c, int& i, int& j, int& k) {
@@ -537,9 +537,9 @@ __device__ __forceinline__ void adj_dir(const AdjArgs& A, unsigned char* smem) {
 template <int DIM, typename S>
 __global__ void __launch_bounds__(kAdjLines * kAdjLen, 2) k_adj_dir(const __grid_constant__ AdjArgs A) {
     extern __shared__ __align__(16) unsigned char smem[];
-    if (blockIdx.y == 0) adj_dir<0, DIM, S>(A, smem);
-    else if (DIM >= 2 && blockIdx.y == 1) adj_dir<(DIM >= 2) ? 1 : 0, DIM, S>(A, smem);
-    else if (DIM >= 3) adj_dir<(DIM >= 3) ? 2 : 0, DIM, S>(A, smem);
+    if (DIM == 1 || blockIdx.x < A.adjFirst[1]) adj_dir<0, DIM, S>(A, smem);
+    else if (DIM == 2 || blockIdx.x < A.adjFirst[2]) adj_dir<(DIM >= 2) ? 1 : 0, DIM, S>(A, smem);
+    else adj_dir<(DIM >= 3) ? 2 : 0, DIM, S>(A, smem);
 }
 
 // ghost images of interior index c along one axis: positions g in the

@@ -18,7 +18,8 @@ struct AdjArgs {
     const double* dtDev;     // non-null: dt is read from device memory (the step's CFL dt)
     const int* skip;         // non-null: the tangent kernels of a skipped step (*skip != 0) do nothing
     int stage0;          // stage 0 of a step: lam += acc0, acc0 = 0
-    unsigned adjTiles;   // blocks along a grid line of the reverse kernel (set by the launcher)
+    unsigned adjFirst[3];   // reverse kernel (set by the launcher): the first block of each direction,
+    unsigned adjTiles[3];   // and the blocks along one of its grid lines
     int fp32;            // local Jacobians of the reverse sweep in FP32
     double* tan[5];      // tangent dU (interior cells)
     double* tan0[5];     // tangent of the step-start state
