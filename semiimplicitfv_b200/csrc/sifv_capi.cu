@@ -618,23 +618,12 @@ int jacobi_run(sifv_ctx* c, const double* rho, const double* rhoc2, const double
     const Params& P = c->P;
     const dim3 g3((unsigned)((P.nx + 31) / 32), (unsigned)((P.ny + 7) / 8), (unsigned)((P.nz + kJacZ - 1) / kJacZ));
     // 3D: two iterations per launch, except with a decomposed mesh, whose
-    // ghost layers and residual are exchanged between the iterations.  The
-    // walk of a segment costs its planes and about three more, and the blocks
-    // run in waves of one per SM: the segment count with the shortest sum.
+    // ghost layers and residual are exchanged between the iterations.
     const bool pairs = P.dim == 3 && !c->exchangeFaces;
     dim3 gp((unsigned)((P.nx + 31) / 32), (unsigned)((P.ny + kJac2Y - 1) / kJac2Y), 1);
     int planes = P.nz;
     if (pairs) {
-        const long long tiles = (long long)gp.x * gp.y, slots = std::max(1, c->jacSms);
-        double best = 0.0;
-        for (int s = 1; s <= P.nz && s <= 64; ++s) {
-            const int n = (P.nz + s - 1) / s;
-            const double cost = (double)((tiles * s + slots - 1) / slots) * (n + 3);
-            if (s == 1 || cost < best) {
-                best = cost;
-                planes = n;
-            }
-        }
+        planes = walk_planes((long long)gp.x * gp.y, std::max(1, c->jacSms), P.nz);   // one block per SM
         gp.z = (unsigned)((P.nz + planes - 1) / planes);
         CUDA_TRY(c, cudaFuncSetAttribute(faceCoef ? k_jacobi3_pair<true> : k_jacobi3_pair<false>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,

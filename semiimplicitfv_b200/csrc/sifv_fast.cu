@@ -130,22 +130,8 @@ int tile3_launch(Tile3Args A, cudaStream_t s) {
         return -1;
     A.tilesX = (A.P.nx + Tile3::TX - 1) / Tile3::TX;
     A.tilesY = (A.P.ny + Tile3::TY - 1) / Tile3::TY;
-    // Segments along z: the walk of a segment costs its planes and about
-    // three planes' worth of start-up, and the blocks run in waves of two per
-    // SM; take the segment count with the shortest sum (down to one plane: a
-    // small mesh is one wave, as long as its longest walk).
-    const long long tiles = (long long)A.tilesX * A.tilesY, slots = 2LL * sms;
-    double best = 0.0;
-    A.segs = 1;
-    for (int g = 1; g <= A.P.nz && g <= 64; ++g) {
-        const int planes = (A.P.nz + g - 1) / g;
-        const double cost = (double)((tiles * g + slots - 1) / slots) * (planes + 3);
-        if (g == 1 || cost < best) {
-            best = cost;
-            A.segs = g;
-        }
-    }
-    A.segPlanes = (A.P.nz + A.segs - 1) / A.segs;
+    const long long tiles = (long long)A.tilesX * A.tilesY;
+    A.segPlanes = walk_planes(tiles, 2LL * sms, A.P.nz);   // two blocks per SM
     A.segs = (A.P.nz + A.segPlanes - 1) / A.segPlanes;
     const long long grid = tiles * A.segs;
     if (grid > 0x7fffffffLL) return -1;
