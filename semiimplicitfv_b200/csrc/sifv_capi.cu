@@ -582,6 +582,26 @@ int launch_chained(sifv_ctx* c, void (*kernel)(KArgs...), dim3 grid, unsigned th
     return launch_chained_smem(c, kernel, grid, threads, 0, args...);
 }
 
+// Whether two 3D iterations in one launch (k_jacobi3_pair, whose blocks take
+// `walk` planes in all, one after the other) take less time than two launches
+// of k_jacobi3 (`blocks` blocks, three per SM, up to 32 planes each).  Times
+// in us per plane and launch as they fit 68 meshes of 8^3 to 200^3 cells and
+// of columns, slabs and bars down to 4 cells wide.  The pair wins by 1.2 to
+// 4.3 where the walks are long or the mesh is one wave (64^3 27.7 -> 8.9 us
+// per iteration), and loses where many tiles have few planes (8000 x 4 x 4
+// 7.7 against 11.5, 4 x 8000 x 4 17.6 against 25.4).  With coefficients per
+// cell, twice the arrays, its one block per SM does not hide the latency of
+// device memory: it wins while they stay in L2 (96^3 41.0 -> 24.7; 112^3 is
+// even, 128^3 57.8 against 61.0, 256^3 302 against 411) or a tile holds whole
+// rows (25 x 256 x 256 59 -> 43).
+bool jacobi_pairs(const sifv_ctx* c, long long walk, long long blocks, bool faceCoef) {
+    const long long slots = 3LL * std::max(1, c->jacSms);
+    const double planes1 = (double)((blocks + slots - 1) / slots) * std::min(c->P.nz, kJacZ);
+    if (faceCoef) return 1.5 * walk + 6.0 <= 2.0 * (1.15 * planes1 + 4.0);
+    const bool inL2 = c->ncells <= 1200000;   // 11 arrays and the halos' second reads, 126 MB
+    return 2.0 * walk + 6.0 <= 2.0 * (1.2 * planes1 + 4.0) && (inL2 || c->P.nx <= 32);
+}
+
 // Jacobi iterations on (rho, rhoc2, rhs) with initial guess in F.pA;
 // returns the number of iterations as JacobiPressureSolver::solve does and
 // the buffer holding the result.
@@ -619,11 +639,15 @@ int jacobi_run(sifv_ctx* c, const double* rho, const double* rhoc2, const double
     const dim3 g3((unsigned)((P.nx + 31) / 32), (unsigned)((P.ny + 7) / 8), (unsigned)((P.nz + kJacZ - 1) / kJacZ));
     // 3D: two iterations per launch, except with a decomposed mesh, whose
     // ghost layers and residual are exchanged between the iterations.
-    const bool pairs = P.dim == 3 && !c->exchangeFaces;
     dim3 gp((unsigned)((P.nx + 31) / 32), (unsigned)((P.ny + kJac2Y - 1) / kJac2Y), 1);
     int planes = P.nz;
+    bool pairs = P.dim == 3 && !c->exchangeFaces;
     if (pairs) {
-        planes = walk_planes((long long)gp.x * gp.y, std::max(1, c->jacSms), P.nz);   // one block per SM
+        long long walk = 0;
+        planes = walk_planes((long long)gp.x * gp.y, std::max(1, c->jacSms), P.nz, &walk);   // one block per SM
+        pairs = jacobi_pairs(c, walk, (long long)g3.x * g3.y * g3.z, faceCoef);
+    }
+    if (pairs) {
         gp.z = (unsigned)((P.nz + planes - 1) / planes);
         CUDA_TRY(c, cudaFuncSetAttribute(faceCoef ? k_jacobi3_pair<true> : k_jacobi3_pair<false>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
