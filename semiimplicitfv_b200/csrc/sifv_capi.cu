@@ -1488,6 +1488,36 @@ void flush_advance(sifv_ctx* c) {
     c->advPending = false;
 }
 
+// Whether the fused stage takes less time than the separate kernels, in the
+// reference-ordered mode.  Its blocks of 32 x 8 cells cost much the same
+// whatever part of their 32 columns lies in the mesh and little less with
+// fewer rows, where the separate kernels' time goes with the cells, after a
+// floor of launches.  2D, us per RK3 step as they fit 264 meshes of 4 to 2000
+// columns and 8000 to 4 million cells (single phase / two phases): fused
+// 25 + 0.082 per block + 0.0078 per row of a tile / 40 + 0.155 + 0.0125,
+// separate 85 + 0.66 per 1000 cells / 90 + 1.34; the viscous terms add 12 and
+// 8 % to the first and a quarter and a seventh to the second.  For example
+// 2000 x 2000: 2235 fused against 2578 / 3910 against 5194; 97 x 24742: 1791
+// against 1667 / 3169 against 3307; 33 x 24242: 896 against 607 / 1576 against
+// 1221; 4 x 25000: 479 against 172 / 832 against 253; 24 x 4166: 115 against
+// 160 / 193 against 225.  1D (30 cells per block, a warp per variable): even
+// at 600000 cells (400000: 169 against 184, 1 million: 389 against 378, 2
+// million: 852 against 741), with two phases at 60000 (30000: 70 against 107,
+// 100000: 166 against 143, 200000: 307 against 201).
+constexpr int kStageCells1D = 600000, kStageCells1DPhases = 60000;
+bool stage_pays(const sifv_ctx* c) {
+    const Params& P = c->P;
+    if (P.dim == 1) return P.nx <= (P.nPh ? kStageCells1DPhases : kStageCells1D);
+    const double tilesX = (P.nx + 31) / 32, blocks = tilesX * ((P.ny + 7) / 8), rows = tilesX * P.ny;
+    const double kCells = 1e-3 * P.nx * (double)P.ny;
+    if (P.nPh) {
+        const double t = 0.155 * blocks + 0.0125 * rows;
+        return P.visc ? 1.08 * t <= 88.0 + 1.52 * kCells : t <= 50.0 + 1.34 * kCells;
+    }
+    const double t = 0.082 * blocks + 0.0078 * rows;
+    return P.visc ? 1.12 * t <= 88.0 + 0.83 * kCells : t <= 60.0 + 0.66 * kCells;
+}
+
 // The explicit steps that run as fused stage kernels (sifv_stage.cuh): the
 // reference-ordered mode in 1D and 2D with the five-cell stencils and at most
 // two phases, where nothing runs between the kernels of a stage (IGR, halo
@@ -1503,7 +1533,8 @@ void flush_advance(sifv_ctx* c) {
 constexpr int kStageFastCells = 240000;
 bool fused_stage(const sifv_ctx* c) {
     const Params& P = c->P;
-    const bool mode = c->cfg.precision == SIFV_PREC_FP64 || (c->sweep && P.dim == 1 && P.nx <= kStageFastCells);
+    const bool mode = c->sweep ? P.dim == 1 && P.nx <= kStageFastCells
+                               : c->cfg.precision == SIFV_PREC_FP64 && P.dim <= 2 && stage_pays(c);
     return mode && !c->cfg.semiImplicit && !c->cfg.useIGR && P.dim <= 2 && c->W == 5 &&
            c->nphT <= 2 && c->cfg.RKOrder > 1 && !P.cap && !c->ib.count && !c->F.solid && !c->exchangeFaces &&
            !c->stageHook && P.ngx <= kStageMaxGhost && P.ny <= 8 * 65535;
