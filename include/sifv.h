@@ -457,7 +457,8 @@ int sifv_ensemble_set_field(sifv_ensemble_t* e, int field, const double* packed,
 int sifv_ensemble_get_field(sifv_ensemble_t* e, int field, double* packed, int onDevice);
 /* Advance every instance until its time reaches tEnd or it has taken
  * maxSteps steps in total (<= 0: no step limit).  blockSize 0: the
- * autotuned (or default 256) threads per instance.  timesOut / stepsOut
+ * autotuned threads per instance, or a default taken from the instances'
+ * sizes.  timesOut / stepsOut
  * (nInst entries each, may be NULL) receive each instance's time and step
  * count; *deviceMs the launch's device time.  An instance whose time step
  * comes out non-positive (a blown-up state) stops there and the call

@@ -28,7 +28,7 @@ struct sifv_ensemble {
     std::vector<void*> allocs;
     std::vector<long long> off;
     long long ncells = 0;
-    int blockSize = 512;
+    int blockSize = 256;       // set from the instances' sizes (sifv_ensemble_create)
     std::string err;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 };
@@ -192,12 +192,15 @@ int sifv_ensemble_create(const sifv_config_t* cfg, int nInst, const int* nCells,
         if (cudaStreamSynchronize(e->stream) != cudaSuccess) st = efail(e, SIFV_ERR_CUDA, "upload failed");
     }
     A.order = ord; A.n = nn; A.off = offd;
-    if (cfg->precision == SIFV_PREC_MIXED && e->nphT <= 2) {
-        // Default block size of a mixed run: 512 threads (two instances per SM) unless the longest instance
-        // (cost n^2, steps going with n) would outlast three times an even split of all of them over the GPU's
-        // warps; then 1024, which halves its chain.  40 steps of 400 tubes of 256 - 4096 cells (ratio 4.1):
-        // 6.18 ms at 512, 4.23 at 1024; 400 of 200 - 800 (2.2): 1.50, 1.74; 2048 of 256 - 4096 (0.8), 10 steps:
-        // 5.14, 5.33.  FP64 runs at most 512 and is fastest there (14.2 ms, 25.5 at 256).
+    {
+        // Default block size.  A block never needs more warps than its longest instance has strips: idle ones hold
+        // registers that other instances could use (4096 tubes of 30 - 60 cells, 20 steps, FP64: 6.80 ms at 512
+        // threads, 1.38 at 96).  Below that FP64 takes 256 threads (two or three instances per SM) and mixed
+        // precision 512, and twice as many where the longest instance (cost n^2, steps going with n) would outlast an
+        // even split of all of them over the GPU, since that halves its chain: `ratio` is its share of the work times
+        // twice the SMs.  FP64, ms at 256 and 512: 400 tubes of 256 - 4096 cells (ratio 4.1) 3.04, 1.74; 300 of
+        // 500 - 1500 (2.4) 1.20, 1.06; 400 of 200 - 800 (2.2) 1.28, 1.40; 2048 of 256 - 4096 (0.8) 2.14, 2.57.
+        // Mixed, at 512 and 1024: 0.62, 0.47 / 0.27, 0.30 / 0.37, 0.43 / 0.62, 0.71.
         int sms = 148;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
         double sum = 0.0, top = 0.0;
@@ -206,7 +209,12 @@ int sifv_ensemble_create(const sifv_config_t* cfg, int nInst, const int* nCells,
             sum += w;
             top = std::max(top, w);
         }
-        if (top / 16.0 > 3.0 * sum / (32.0 * sms)) e->blockSize = 1024;
+        const double ratio = 2.0 * sms * top / sum;
+        const bool mixed = cfg->precision == SIFV_PREC_MIXED;
+        const bool wide = ratio > (mixed ? 3.0 : 2.3) && !(mixed && e->nphT > 2);   // 8 phases: no room for 1024
+        const int warps = (mixed ? 16 : 8) * (wide ? 2 : 1);
+        const int strips = (nCells[order[0]] + kEnsStrip - 1) / kEnsStrip;
+        e->blockSize = std::min(32 * std::min(warps, strips), max_block(e));
     }
     Params& P = A.P;
     P.dim = 1; P.ny = P.nz = 1; P.ngx = ng; P.ngy = P.ngz = 0; P.nyT = P.nzT = 1;
