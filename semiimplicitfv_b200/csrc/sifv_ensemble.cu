@@ -28,6 +28,7 @@ struct sifv_ensemble {
     std::vector<void*> allocs;
     std::vector<long long> off;
     long long ncells = 0;
+    int sms = 148;
     int blockSize = 256;       // set from the instances' sizes (sifv_ensemble_create)
     std::string err;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -69,18 +70,54 @@ double* efield(sifv_ensemble* e, int f) {
     return nullptr;
 }
 
-template <typename T, int NPH>
-int launch_t(const EnsArgs& A, int blockSize, cudaStream_t s) {
-    k_ensemble<T, NPH><<<A.nInst, blockSize, 0, s>>>(A);
+// Whether an FP64 run takes the block's chunks (blockDim - 6 cells) or its
+// warps' strips (26 cells each).  An instance's rounds, weighted with its steps
+// (n), are fewer with chunks unless it is short, and a round of chunks costs
+// 8 % more; 30 % more where an SM holds more blocks of strips (one phase: 78
+// registers against 124) and the instances fill at least 0.4 of those places,
+// measured by the longest.  ms, strips and chunks.  Two phases: 2048 instances
+// of 256 - 4096 cells 5.42, 4.89 at 256 threads; 60 of 200 - 1000 1.87, 1.51 at
+// 512; 512 of 30 - 200 1.18, 1.24 at 256; 60 of 200 - 400 0.70, 0.75 at 512.
+// One phase: 60 of 200 - 1000 0.91, 0.75 at 512; 300 of 500 - 1500 1.19, 0.97
+// at 256; 2048 of 256 - 4096 2.14, 2.23 at 256 and 2.31, 3.14 at 320; 148 of
+// 30 - 100 0.27, 0.29.
+template <int NPH>
+bool ensemble_chunks(const sifv_ensemble* e, int blockSize) {
+    const int warps = blockSize / 32, cells = blockSize - 6;
+    double strips = 0.0, chunks = 0.0, top = 0.0;
+    for (int k = 0; k < e->nInst; ++k) {
+        const int n = (int)(e->off[k + 1] - e->off[k]) - 2 * e->A.P.ngx;
+        const double w = (double)n * (((n + kEnsStrip - 1) / kEnsStrip + warps - 1) / warps);
+        strips += w;
+        top = std::max(top, w);
+        chunks += (double)n * ((n + cells - 1) / cells);
+    }
+    int byStrips = 0, byChunks = 0;   // blocks per SM
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&byStrips, k_ensemble<double, NPH, false>, blockSize, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&byChunks, k_ensemble<double, NPH, true>, blockSize, ens_smem<NPH>(blockSize));
+    const bool crowded = byStrips > byChunks && strips >= 0.4 * e->sms * byStrips * top;
+    return chunks * (crowded ? 1.3 : 1.08) < strips;
+}
+
+template <int NPH>
+int launch_d(const sifv_ensemble* e, int blockSize) {
+    const size_t bytes = ens_smem<NPH>(blockSize);
+    if (cudaFuncSetAttribute(k_ensemble<double, NPH, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) !=
+        cudaSuccess)
+        return -1;
+    if (ensemble_chunks<NPH>(e, blockSize))
+        k_ensemble<double, NPH, true><<<e->nInst, blockSize, bytes, e->stream>>>(e->A);
+    else
+        k_ensemble<double, NPH, false><<<e->nInst, blockSize, 0, e->stream>>>(e->A);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
 int launch(sifv_ensemble* e, int blockSize) {
     if (e->cfg.precision == SIFV_PREC_MIXED)
         return ensemble_launch_mixed(e->A, e->nphT, blockSize, e->stream);
-    if (e->nphT == 0) return launch_t<double, 0>(e->A, blockSize, e->stream);
-    if (e->nphT == 2) return launch_t<double, 2>(e->A, blockSize, e->stream);
-    return launch_t<double, 8>(e->A, blockSize, e->stream);
+    if (e->nphT == 0) return launch_d<0>(e, blockSize);
+    if (e->nphT == 2) return launch_d<2>(e, blockSize);
+    return launch_d<8>(e, blockSize);
 }
 
 // the largest usable block size
@@ -201,15 +238,14 @@ int sifv_ensemble_create(const sifv_config_t* cfg, int nInst, const int* nCells,
         // twice the SMs.  FP64, ms at 256 and 512: 400 tubes of 256 - 4096 cells (ratio 4.1) 3.04, 1.74; 300 of
         // 500 - 1500 (2.4) 1.20, 1.06; 400 of 200 - 800 (2.2) 1.28, 1.40; 2048 of 256 - 4096 (0.8) 2.14, 2.57.
         // Mixed, at 512 and 1024: 0.62, 0.47 / 0.27, 0.30 / 0.37, 0.43 / 0.62, 0.71.
-        int sms = 148;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+        cudaDeviceGetAttribute(&e->sms, cudaDevAttrMultiProcessorCount, device);
         double sum = 0.0, top = 0.0;
         for (int k = 0; k < nInst; ++k) {
             const double w = (double)nCells[k] * nCells[k];
             sum += w;
             top = std::max(top, w);
         }
-        const double ratio = 2.0 * sms * top / sum;
+        const double ratio = 2.0 * e->sms * top / sum;
         const bool mixed = cfg->precision == SIFV_PREC_MIXED;
         const bool wide = ratio > (mixed ? 3.0 : 2.3) && !(mixed && e->nphT > 2);   // 8 phases: no room for 1024
         const int warps = (mixed ? 16 : 8) * (wide ? 2 : 1);

@@ -12,10 +12,14 @@
 // of its cell from the neighbours' primitives (shuffles), solves the Riemann
 // problem at its high face with the next lane's value, and updates its cell
 // from its own and the previous lane's flux.  Warps of a stage share nothing:
-// the block synchronises once per stage.  (Chunks of the whole block in
-// shared memory, with four barriers per chunk of blockDim - 6 cells, left the
-// block waiting for the longest chain of each phase: 400 tubes of 256 to
-// 4096 cells, 40 steps in mixed precision, 14.7 ms; now 4.3 ms.)
+// the block synchronises once per stage.  (Mixed precision, 400 tubes of 256
+// to 4096 cells, 40 steps: 4.3 ms, where chunks of the whole block in shared
+// memory took 14.7.)  With CHUNKS, FP64 only, the team that shares a halo is
+// the block instead: blockDim - 6 cells at a time, values passed through
+// shared memory between three barriers.  Of 32 lanes a strip leaves 6 to the
+// halo, and FP64 arithmetic is the bound on long instances (20 % of it the
+// halo's); the barriers are the price, and short instances leave more of a
+// block idle than of a warp (ensemble_chunks, sifv_ensemble.cu).
 // The stage input and output are different packed states (S[0] the state,
 // S[1], S[2] scratch; the last stage writes S[0], which only the cell itself
 // reads there as U0), so strips never see each other's updates.  The last
@@ -187,8 +191,16 @@ __device__ __forceinline__ double ens_limit(const EnsArgs& A, const Params& P, l
 
 constexpr int kEnsStrip = 26;   // cells per warp and strip: 32 lanes less a three-cell halo on either side
 
-template <typename T, int NPH>
+// Shared memory of a block with CHUNKS (FP64): per thread the primitives, the
+// low-face values, the mass fractions and the fluxes.
+template <int NPH>
+__host__ __device__ constexpr size_t ens_smem(int threads) {
+    return sizeof(double) * threads * (2 * (3 + NPH) + NPH + 3 + ((NPH > 0) ? 1 + 2 * NPH : 0));
+}
+
+template <typename T, int NPH, bool CHUNKS>
 __global__ void __launch_bounds__(EnsMaxThreads<T, NPH>::value) k_ensemble(const __grid_constant__ EnsArgs A) {
+    extern __shared__ __align__(16) unsigned char ensSmem[];   // CHUNKS: ens_smem()
     __shared__ double red[33];
     constexpr int NVR = 3 + NPH;       // reconstructed: rho, u, p, alpha[NPH]
     constexpr unsigned kAll = 0xffffffffu;
@@ -261,112 +273,179 @@ __global__ void __launch_bounds__(EnsMaxThreads<T, NPH>::value) k_ensemble(const
             const EnsState& Out = (lastStage && RK > 1) ? A.S[0] : A.S[s + 1];
             const bool writePrim = lastStage && RK > 1;
 
-            for (int c0 = warp * kEnsStrip; c0 < n; c0 += nWarps * kEnsStrip) {
-                // ---- primitives of position q (lanes past the last ghost repeat it) ----
-                const int q = c0 - 3 + lane;
-                double sn, sa;
-                const int sq = prim_src(min(q, n + 2), n, P.bc[0], P.bc[1], sn, sa);
-                const long long c = at(sq);
-                double rhoP, u, p, ar[NPH > 0 ? NPH : 1], al[NPH > 0 ? NPH : 1];
-#pragma unroll
-                for (int ph = 0; ph < NPH; ++ph) {
-                    ar[ph] = (ph < P.nPh) ? In.alphaRho[ph][c] : 0.0;
-                    al[ph] = (ph < P.nPh) ? In.alpha[ph][c] : 0.0;
-                }
-                const double mom = In.rhoU[c], rhoE = In.rhoE[c];
-                ens_prim<T, NPH>(A, P, (NPH > 0) ? 0.0 : In.rho[c], mom, rhoE, ar, al, rhoP, u, p);
+            // a team of consecutive threads takes its cells and a halo of three on either side: a warp, or the block
+            const int team = CHUNKS ? (int)blockDim.x : 32, me = CHUNKS ? (int)threadIdx.x : lane;
+            T* const sW = reinterpret_cast<T*>(ensSmem);
+            T* const sLo = sW + NVR * team;
+            double* const sY = reinterpret_cast<double*>(sLo + NVR * team);
+            double* const sF = sY + NPH * team;
+            const int first = CHUNKS ? 0 : warp * kEnsStrip, step = CHUNKS ? team - 6 : nWarps * kEnsStrip;
+            for (int c0 = first; c0 < n; c0 += step) {
+                // ---- primitives of position q (threads past the last ghost repeat it) ----
+                const int q = c0 - 3 + me;
+                // a block's warps past the last ghost have nothing to do but the barriers
+                const bool live = !CHUNKS || q - lane < n + 3;
+                long long c = 0;
+                double mom = 0.0, rhoE = 0.0, rhoP = 0.0, ar[NPH > 0 ? NPH : 1], al[NPH > 0 ? NPH : 1];
+                double y[NPH > 0 ? NPH : 1];   // mass fractions
                 T w[NVR], hi[NVR], lo[NVR];
-                w[0] = T(rhoP);
-                w[1] = T((sn * sa) * u);
-                w[2] = T(p);
-#pragma unroll
-                for (int ph = 0; ph < NPH; ++ph) w[3 + ph] = T(al[ph]);
-                // ---- both face values of the cell (lanes 2 .. 29) ----
-#pragma unroll
-                for (int v = 0; v < NVR; ++v) {
-                    if (v >= 3 && v - 3 >= P.nPh) continue;
-                    const T x0 = __shfl_up_sync(kAll, w[v], 2), x1 = __shfl_up_sync(kAll, w[v], 1);
-                    const T x3 = __shfl_down_sync(kAll, w[v], 1), x4 = __shfl_down_sync(kAll, w[v], 2);
-                    if (weno) {
-                        if constexpr (sizeof(T) == 4) {
-                            weno5_pair(x0, x1, w[v], x3, x4, T(eps), hi[v], lo[v]);
-                        } else {
-                            hi[v] = weno5_high<T>(x0, x1, w[v], x3, x4, T(eps));
-                            lo[v] = weno5_low<T>(x0, x1, w[v], x3, x4, T(eps));
-                        }
-                    } else {
-                        hi[v] = upwind5L<T>(x0, x1, w[v], x3, x4);
-                        lo[v] = upwind5R<T>(x0, x1, w[v], x3, x4);
-                    }
-                }
-                // ---- the cell's high face (lanes 2 .. 28): left state its own, right state the next lane's ----
-                FaceState<NPH, T> L, R;
-                L.u[1] = L.u[2] = R.u[1] = R.u[2] = T(0.0);
-                L.sigma = R.sigma = T(0.0);
-                L.rho = hi[0];
-                L.u[0] = hi[1];
-                L.p = hi[2];
-                R.rho = __shfl_down_sync(kAll, lo[0], 1);
-                R.u[0] = __shfl_down_sync(kAll, lo[1], 1);
-                R.p = __shfl_down_sync(kAll, lo[2], 1);
-#pragma unroll
-                for (int ph = 0; ph < NPH; ++ph) {
-                    L.alpha[ph] = R.alpha[ph] = T(0.0);
-                    if (ph < P.nPh) {
-                        L.alpha[ph] = hi[3 + ph];
-                        R.alpha[ph] = __shfl_down_sync(kAll, lo[3 + ph], 1);
-                    }
-                }
-                if (NPH > 0) {
-                    eff_gamma_piinf<NPH, T>(P, L.alpha, L.gEff, L.piEff);
-                    eff_gamma_piinf<NPH, T>(P, R.alpha, R.gEff, R.piEff);
-                } else {
-                    L.gEff = R.gEff = T(P.gamma);
-                    L.piEff = R.piEff = T(P.pInf);
-                }
-                FaceFlux<NPH, T> Fx;
-                switch (P.riemann) {
-                    case SIFV_HLLC: hllc_flux<0, NPH, T>(P, L, R, Fx); break;
-                    case SIFV_RUSANOV: rusanov_flux<0, NPH, T>(P, L, R, Fx); break;
-                    default: lf_flux<0, NPH, T>(P, L, R, Fx); break;
-                }
-                __syncwarp();
-                // upwinded partial-density flux (src/ExplicitSolver.cpp:307-326)
-                double fAR[NPH > 0 ? NPH : 1];
-                if (NPH > 0) {
-                    const double iRho = (sizeof(T) == 8) ? 0.0 : frcp(smax(rhoP, 1e-14));
+                if (live) {
+                    double sn, sa, u, p;
+                    const int sq = prim_src(min(q, n + 2), n, P.bc[0], P.bc[1], sn, sa);
+                    c = at(sq);
 #pragma unroll
                     for (int ph = 0; ph < NPH; ++ph) {
+                        ar[ph] = (ph < P.nPh) ? In.alphaRho[ph][c] : 0.0;
+                        al[ph] = (ph < P.nPh) ? In.alpha[ph][c] : 0.0;
+                    }
+                    mom = In.rhoU[c];
+                    rhoE = In.rhoE[c];
+                    ens_prim<T, NPH>(A, P, (NPH > 0) ? 0.0 : In.rho[c], mom, rhoE, ar, al, rhoP, u, p);
+                    w[0] = T(rhoP);
+                    w[1] = T((sn * sa) * u);
+                    w[2] = T(p);
+#pragma unroll
+                    for (int ph = 0; ph < NPH; ++ph) w[3 + ph] = T(al[ph]);
+                    if constexpr (CHUNKS) {
+#pragma unroll
+                        for (int v = 0; v < NVR; ++v) sW[v * team + me] = w[v];
+                    }
+                }
+                if constexpr (CHUNKS) __syncthreads();
+                // ---- both face values of the cell (all but the outer two threads) ----
+                if (live) {
+#pragma unroll
+                    for (int v = 0; v < NVR; ++v) {
+                        if (v >= 3 && v - 3 >= P.nPh) continue;
+                        T x0, x1, x3, x4;
+                        if constexpr (CHUNKS) {
+                            const T* const x = sW + v * team + min(max(me, 2), team - 3);
+                            x0 = x[-2]; x1 = x[-1]; x3 = x[1]; x4 = x[2];
+                        } else {
+                            x0 = __shfl_up_sync(kAll, w[v], 2); x1 = __shfl_up_sync(kAll, w[v], 1);
+                            x3 = __shfl_down_sync(kAll, w[v], 1); x4 = __shfl_down_sync(kAll, w[v], 2);
+                        }
+                        if (weno) {
+                            if constexpr (sizeof(T) == 4) {
+                                weno5_pair(x0, x1, w[v], x3, x4, T(eps), hi[v], lo[v]);
+                            } else {
+                                hi[v] = weno5_high<T>(x0, x1, w[v], x3, x4, T(eps));
+                                lo[v] = weno5_low<T>(x0, x1, w[v], x3, x4, T(eps));
+                            }
+                        } else {
+                            hi[v] = upwind5L<T>(x0, x1, w[v], x3, x4);
+                            lo[v] = upwind5R<T>(x0, x1, w[v], x3, x4);
+                        }
+                        if constexpr (CHUNKS) sLo[v * team + me] = lo[v];
+                    }
+                    if constexpr (CHUNKS && NPH > 0) {
+#pragma unroll
+                        for (int ph = 0; ph < NPH; ++ph)
+                            if (ph < P.nPh) sY[ph * team + me] = y[ph] = ar[ph] / smax(rhoP, 1e-14);
+                    }
+                }
+                if constexpr (CHUNKS) __syncthreads();
+                // ---- the cell's high face: left state its own, right state the next thread's ----
+                FaceFlux<NPH, T> Fx;
+                double fAR[NPH > 0 ? NPH : 1];
+                if (live) {
+                    const int next = CHUNKS ? min(me + 1, team - 1) : 0;
+                    auto above = [&](int v) -> T {
+                        if constexpr (CHUNKS) return sLo[v * team + next];
+                        else return __shfl_down_sync(kAll, lo[v], 1);
+                    };
+                    FaceState<NPH, T> L, R;
+                    L.u[1] = L.u[2] = R.u[1] = R.u[2] = T(0.0);
+                    L.sigma = R.sigma = T(0.0);
+                    L.rho = hi[0];
+                    L.u[0] = hi[1];
+                    L.p = hi[2];
+                    R.rho = above(0);
+                    R.u[0] = above(1);
+                    R.p = above(2);
+#pragma unroll
+                    for (int ph = 0; ph < NPH; ++ph) {
+                        L.alpha[ph] = R.alpha[ph] = T(0.0);
                         if (ph < P.nPh) {
-                            const double y = (sizeof(T) == 8) ? ar[ph] / smax(rhoP, 1e-14) : ar[ph] * iRho;
-                            const double yr = __shfl_down_sync(kAll, y, 1);
-                            fAR[ph] = (((double)Fx.mass >= 0) ? y : yr) * (double)Fx.mass;
+                            L.alpha[ph] = hi[3 + ph];
+                            R.alpha[ph] = above(3 + ph);
+                        }
+                    }
+                    if (NPH > 0) {
+                        eff_gamma_piinf<NPH, T>(P, L.alpha, L.gEff, L.piEff);
+                        eff_gamma_piinf<NPH, T>(P, R.alpha, R.gEff, R.piEff);
+                    } else {
+                        L.gEff = R.gEff = T(P.gamma);
+                        L.piEff = R.piEff = T(P.pInf);
+                    }
+                    switch (P.riemann) {
+                        case SIFV_HLLC: hllc_flux<0, NPH, T>(P, L, R, Fx); break;
+                        case SIFV_RUSANOV: rusanov_flux<0, NPH, T>(P, L, R, Fx); break;
+                        default: lf_flux<0, NPH, T>(P, L, R, Fx); break;
+                    }
+                    __syncwarp();
+                    // upwinded partial-density flux (src/ExplicitSolver.cpp:307-326)
+                    if (NPH > 0) {
+                        const double iRho = (sizeof(T) == 8) ? 0.0 : frcp(smax(rhoP, 1e-14));
+#pragma unroll
+                        for (int ph = 0; ph < NPH; ++ph) {
+                            if (ph < P.nPh) {
+                                double yr;
+                                if constexpr (CHUNKS) {
+                                    yr = sY[ph * team + next];
+                                } else {
+                                    y[ph] = (sizeof(T) == 8) ? ar[ph] / smax(rhoP, 1e-14) : ar[ph] * iRho;
+                                    yr = __shfl_down_sync(kAll, y[ph], 1);
+                                }
+                                fAR[ph] = (((double)Fx.mass >= 0) ? y[ph] : yr) * (double)Fx.mass;
+                            }
+                        }
+                    }
+                    if constexpr (CHUNKS) {
+                        sF[me] = Fx.mass;
+                        sF[team + me] = Fx.mom[0];
+                        sF[2 * team + me] = Fx.energy;
+                        if (NPH > 0) {
+                            sF[3 * team + me] = Fx.fvel;
+#pragma unroll
+                            for (int ph = 0; ph < NPH; ++ph)
+                                if (ph < P.nPh) {
+                                    sF[(4 + ph) * team + me] = Fx.alpha[ph];
+                                    sF[(4 + NPH + ph) * team + me] = fAR[ph];
+                                }
                         }
                     }
                 }
-                // ---- the cell (lanes 3 .. 28): divergence (src/ExplicitSolver.cpp:294-496) + update (127-188) ----
-                const bool mine = lane >= 3 && lane <= 28 && q < n;
+                if constexpr (CHUNKS) __syncthreads();
+                // ---- the cell (all but the outer three threads): divergence (src/ExplicitSolver.cpp:294-496) and
+                // update (127-188) ----
+                const bool mine = me >= 3 && me < team - 3 && q < n;
+                if (CHUNKS && !mine) continue;
                 const double dx = A.dx[c];
                 const double coeff = ens_div<T>(1.0 * 1.0, (dx * 1.0) * 1.0);
-                auto div = [&](double f) {
-                    const double fl = __shfl_up_sync(kAll, f, 1);
+                auto below = [&](double f, int row) {   // the flux through the cell's low face
+                    if constexpr (CHUNKS) return sF[row * team + me - 1];
+                    else return __shfl_up_sync(kAll, f, 1);
+                };
+                auto div = [&](double f, int row) {
+                    const double fl = below(f, row);
                     double r = 0.0;
                     r += coeff * fl;
                     r -= coeff * f;
                     return r;
                 };
-                const double rR = div((double)Fx.mass), rU = div((double)Fx.mom[0]), rE = div((double)Fx.energy);
+                const double rR = div((double)Fx.mass, 0), rU = div((double)Fx.mom[0], 1), rE = div((double)Fx.energy, 2);
                 double rAR[NPH > 0 ? NPH : 1], rA[NPH > 0 ? NPH : 1];
                 if (NPH > 0) {
-                    const double fl = __shfl_up_sync(kAll, (double)Fx.fvel, 1);
+                    const double fl = below((double)Fx.fvel, 3);
                     double divU = 0.0;
                     divU -= coeff * fl;
                     divU += coeff * (double)Fx.fvel;
 #pragma unroll
                     for (int ph = 0; ph < NPH; ++ph) {
                         if (ph < P.nPh) {
-                            rAR[ph] = div(fAR[ph]);
-                            double r2 = div((double)Fx.alpha[ph]);
+                            rAR[ph] = div(fAR[ph], 4 + NPH + ph);
+                            double r2 = div((double)Fx.alpha[ph], 4 + ph);
                             r2 += al[ph] * divU;
                             rA[ph] = r2;
                         }

@@ -12,7 +12,7 @@ namespace sifv {
 namespace {
 template <int NPH>
 int launch_f(const EnsArgs& A, int blockSize, cudaStream_t s) {
-    k_ensemble<float, NPH><<<A.nInst, blockSize, 0, s>>>(A);
+    k_ensemble<float, NPH, false><<<A.nInst, blockSize, 0, s>>>(A);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 }  // namespace
