@@ -560,9 +560,10 @@ int igr_solve(sifv_ctx* c, int step) {
 }
 
 // A kernel of a chain whose every kernel waits for the one before it
-// (grid_dep_wait): set up while that one still runs.
+// (grid_dep_wait): set up while that one still runs (early), or after it.
 template <typename... KArgs, typename... Args>
-int launch_chained_smem(sifv_ctx* c, void (*kernel)(KArgs...), dim3 grid, unsigned threads, size_t smem, Args... args) {
+int launch_chained_smem(sifv_ctx* c, void (*kernel)(KArgs...), dim3 grid, unsigned threads, size_t smem, bool early,
+                        Args... args) {
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
@@ -572,14 +573,14 @@ int launch_chained_smem(sifv_ctx* c, void (*kernel)(KArgs...), dim3 grid, unsign
     lc.dynamicSmemBytes = smem;
     lc.stream = c->stream;
     lc.attrs = at;
-    lc.numAttrs = 1;
+    lc.numAttrs = early ? 1 : 0;
     CUDA_TRY(c, cudaLaunchKernelEx(&lc, kernel, KArgs(args)...));
     c->launches++;
     return SIFV_OK;
 }
 template <typename... KArgs, typename... Args>
 int launch_chained(sifv_ctx* c, void (*kernel)(KArgs...), dim3 grid, unsigned threads, Args... args) {
-    return launch_chained_smem(c, kernel, grid, threads, 0, args...);
+    return launch_chained_smem(c, kernel, grid, threads, 0, true, args...);
 }
 
 // Whether two 3D iterations in one launch (k_jacobi3_pair, whose blocks take
@@ -655,10 +656,18 @@ int jacobi_run(sifv_ctx* c, const double* rho, const double* rhoc2, const double
     }
     double* const buf[2] = {c->F.pA, c->F.pB};
     int launched = 0;   // an iteration or a pair reads buf[launched % 2] and writes the other
+    // The early blocks of a 3D iteration that wait on an SM take it from no
+    // one where half the SMs are free, and are the next wave where three
+    // waves' worth are queued.  In between they end up two on one SM beside
+    // idle ones, which costs more than the launch unless the walks are short
+    // (us early / after: 96^3 32.9 / 29.5, 112^3 40.1 / 34.9, 9 x 256 x 256
+    // 39.4 / 33.2; 64^3 27.6 / 29.0, 256 x 256 x 4 9.2 / 10.4, 200^3 125 / 127).
+    const long long blocks3 = (long long)g3.x * g3.y * g3.z;
+    const bool early3 = 2 * blocks3 <= c->jacSms || blocks3 >= 3LL * c->jacSms || std::min(P.nz, kJacZ) <= 9;
     auto single = [&](int n, const double* pin, double* pout) {
         if (P.dim == 3)
-            return launch_chained(c, faceCoef ? k_jacobi3<true> : k_jacobi3<false>, g3, 256, P,
-                                  (const double*)c->jacCoef, c->ncells, rhoc2, rhs, pin, pout, c->ctl, n, tol);
+            return launch_chained_smem(c, faceCoef ? k_jacobi3<true> : k_jacobi3<false>, g3, 256, 0, early3, P,
+                                       (const double*)c->jacCoef, c->ncells, rhoc2, rhs, pin, pout, c->ctl, n, tol);
         if (faceCoef)
             return launch_chained(c, k_jacobi_face, dim3(gj), kCellThreads, P, (const double*)c->jacCoef, c->ncells, rhoc2,
                                   rhs, pin, pout, c->ctl, n, tol);
@@ -675,7 +684,7 @@ int jacobi_run(sifv_ctx* c, const double* rho, const double* rhoc2, const double
             double* pout = buf[(launched & 1) ^ 1];
             if (pairs && it + 2 <= end) {
                 st = launch_chained_smem(c, faceCoef ? k_jacobi3_pair<true> : k_jacobi3_pair<false>, gp, kJac2Threads,
-                                         faceCoef ? jac2_smem<true>() : jac2_smem<false>(), P, (const double*)c->jacCoef,
+                                         faceCoef ? jac2_smem<true>() : jac2_smem<false>(), true, P, (const double*)c->jacCoef,
                                          c->ncells, rhoc2, rhs, pin, pout, c->ctl, it, tol, planes);
                 if (st != SIFV_OK) return st;
                 it += 2;
