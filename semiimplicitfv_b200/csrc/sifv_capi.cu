@@ -66,6 +66,7 @@ struct sifv_ctx {
     std::vector<std::pair<std::string, cudaEvent_t>> marks;
     // fused sweep path (SIFV_PREC_MIXED / SIFV_PREC_FP64_FAST)
     bool sweep = false;
+    bool lines3d = false;                     // a 3D step of dimension sweeps (sweeps_3d)
     double* rhsBuf[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     double* invW[3] = {nullptr, nullptr, nullptr};
     double* rhoP = nullptr;
@@ -1551,7 +1552,7 @@ bool fused_stage(const sifv_ctx* c) {
 
 // Whether the step's last stage folds the next step's dt limits into
 // ctl->dtBits.
-bool folds_dt(const sifv_ctx* c) { return (c->sweep && c->P.dim >= 2) || fused_stage(c); }
+bool folds_dt(const sifv_ctx* c) { return (c->sweep && c->P.dim >= 2 && !c->lines3d) || fused_stage(c); }
 
 int enqueue_dt(sifv_ctx* c, double targetDt, int useEnd) {
     const sifv_config_t& cfg = c->cfg;
@@ -1771,7 +1772,7 @@ int enqueue_step(sifv_ctx* c, int step, double time, double targetDt, int useEnd
         c->dtReady = cfg.constDt <= 0 && c->forcedDt <= 0;
         return SIFV_OK;
     }
-    if (c->sweep && P.dim == 3) {
+    if (c->sweep && P.dim == 3 && !c->lines3d) {
         double* U[5] = {c->F.rho, c->F.rhoU, c->F.rhoV, c->F.rhoW, c->F.rhoE};
         const int RK = cfg.RKOrder;
         const bool fold = cfg.constDt <= 0 && c->forcedDt <= 0;
@@ -2174,11 +2175,15 @@ int sifv_create(const sifv_config_t* cfg, const sifv_mesh_t* mesh, int device, s
     F.dx = g[0]; F.dy = g[1]; F.dz = g[2]; F.adx2 = g[3]; F.ady2 = g[4]; F.adz2 = g[5];
     if (cfg->precision != SIFV_PREC_FP64 && !cfg->semiImplicit) {
         c->sweep = true;
-        if (dim == 1 && !fused_stage(c)) {
+        if (dim == 3) {
+            int sms = 0;
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+            c->lines3d = sweeps_3d(P, cfg->precision == SIFV_PREC_MIXED, sms);
+        }
+        if ((dim == 1 && !fused_stage(c)) || c->lines3d) {
             c->rhoP = dalloc(c, n, st);
-            c->rhsBuf[0] = dalloc(c, n, st);
-            c->rhsBuf[1] = dalloc(c, n, st);
-            c->rhsBuf[4] = dalloc(c, n, st);
+            for (int q = 0; q < 5; ++q)
+                if (dim == 3 || q < 2 || q == 4) c->rhsBuf[q] = dalloc(c, n, st);
         }
         const std::vector<double>* w[3] = {&dxv, &dyv, &dzv};
         for (int a = 0; a < 3; ++a) {
@@ -2192,7 +2197,8 @@ int sifv_create(const sifv_config_t* cfg, const sifv_mesh_t* mesh, int device, s
         if (st == SIFV_OK) cudaStreamSynchronize(c->stream);   // host vectors above go out of scope
     }
     if (st == SIFV_OK) st = ensure_res(c, std::max(cfg->maxPressureIters, 1));
-    if (st == SIFV_OK) st = fused_stage(c) ? stage_buffers(c) : (c->sweep && dim >= 2) ? tile_buffers(c) : split_buffers(c);
+    if (st == SIFV_OK) st = fused_stage(c) ? stage_buffers(c)
+                               : (c->sweep && dim >= 2 && !c->lines3d) ? tile_buffers(c) : split_buffers(c);
     if (st == SIFV_OK) {
         cudaError_t e = cudaStreamSynchronize(c->stream);
         if (e != cudaSuccess) st = fail(c, SIFV_ERR_CUDA, cudaGetErrorString(e));

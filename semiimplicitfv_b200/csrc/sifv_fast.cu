@@ -5,6 +5,8 @@
 // equality.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cmath>
 #include <cstring>
 
 #include "sifv_sweep.cuh"
@@ -16,26 +18,41 @@ namespace sifv {
 
 namespace {
 
+constexpr int kSegment = 32;    // cells per thread along y / z
 constexpr int kSegmentX = 510;  // cells per warp along x: 16 steps of 32 positions
 
-template <typename T>
-int stage_1d(const SweepArgs& A, cudaStream_t s, int& launches, LaunchMark mark, void* user) {
+template <int DIM, typename T>
+int stage_dim(const SweepArgs& A, cudaStream_t s, int& launches, LaunchMark mark, void* user) {
     const Params& P = A.P;
-    long long warps = (P.nx + A.segx - 1) / A.segx;
-    k_sweep_x<1, T><<<(unsigned)((warps + 3) / 4), 128, 0, s>>>(A);
-    ++launches;
-    if (mark) mark(user, "sweep_x");
-    k_rk_update<1><<<(unsigned)(((long long)P.nx + 255) / 256), 256, 0, s>>>(A);
-    ++launches;
-    if (mark) mark(user, "rk_update");
+    auto done = [&](const char* family) {
+        ++launches;
+        if (mark) mark(user, family);
+    };
+    const long long warps = (long long)P.ny * P.nz * ((P.nx + A.segx - 1) / A.segx);
+    k_sweep_x<DIM, T><<<(unsigned)((warps + 3) / 4), 128, 0, s>>>(A);
+    done("sweep_x");
+    if constexpr (DIM == 1) {
+        k_rk_update<<<(unsigned)(((long long)P.nx + 255) / 256), 256, 0, s>>>(A);
+        done("rk_update");
+    } else {
+        const dim3 gy((P.nx + 127) / 128, (P.ny + A.seg - 1) / A.seg, P.nz);
+        k_sweep_line<1, T, false><<<gy, 128, 0, s>>>(A);
+        done("sweep_y");
+        const dim3 gz((P.nx + 127) / 128, (P.nz + A.seg - 1) / A.seg, P.ny);
+        k_sweep_line<2, T, true><<<gz, 128, 0, s>>>(A);
+        done("sweep_z");
+    }
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
 }  // namespace
 
 int sweep_stage(SweepArgs A, cudaStream_t s, bool mixed, int& launches, LaunchMark mark, void* user) {
+    A.seg = kSegment;
     A.segx = kSegmentX;
-    return mixed ? stage_1d<float>(A, s, launches, mark, user) : stage_1d<double>(A, s, launches, mark, user);
+    if (A.P.dim == 1)
+        return mixed ? stage_dim<1, float>(A, s, launches, mark, user) : stage_dim<1, double>(A, s, launches, mark, user);
+    return mixed ? stage_dim<3, float>(A, s, launches, mark, user) : stage_dim<3, double>(A, s, launches, mark, user);
 }
 
 namespace {
@@ -158,6 +175,37 @@ int tile3_dispatch(const Tile3Args& A, cudaStream_t s) {
 }
 
 }  // namespace
+
+// Times of an RK3 step in us as they fit 110 meshes of 3 to 200000 cells per
+// axis (mean error 8 %).  The sweeps cost the steps of their warps: 32
+// positions of a row at a time and three more per segment of 510 to start, or
+// one cell of 32 lines at a time and four more per segment of 32; and the
+// launches and the dt pass.  The tiles cost the planes their blocks walk, in
+// waves (w) and on average (q), more with more of the eight rows in use.  What
+// decides is mostly how well tiles of 8 rows fit ny: us per step, tiles and
+// sweeps, FP64 / mixed: 300 x 9 x 300 783, 552 / 525, 466; 300 x 17 x 300 1202,
+// 983 / 797, 738; 9 x 9 x 30000 6515, 4594 / 4431, 3396; 200000 x 4 x 4 2698,
+// 1903 / 2002, 1577; the other way 300 x 8 x 300 428, 522 / 292, 436; 64^3 180,
+// 395 / 128, 335.  Large FP64 meshes are near even: 203 x 160 x 131 2276, 2189,
+// 130^3 1536, 1556 (mixed 1501, 1788; 1017, 1241).  FP64 takes the sweeps where
+// they are estimated 6 % shorter.
+bool sweeps_3d(const Params& P, bool mixed, int sms) {
+    if (P.ny > 65535 || P.nz > 65535) return false;   // grid limits of the line sweeps
+    const double nx = P.nx, ny = P.ny, nz = P.nz;
+    auto parts = [](int n, int size) { return (double)((n + size - 1) / size); };
+    const double segsX = parts(P.nx, kSegmentX), warps = parts(P.nx, 32);
+    const double x = 1e-3 * ny * nz * (std::ceil((nx + 2.0 * segsX) / 32.0) + 3.0 * segsX);
+    const double y = 1e-3 * warps * nz * (ny + 4.0 * parts(P.ny, kSegment));
+    const double z = 1e-3 * warps * ny * (nz + 4.0 * parts(P.nz, kSegment));
+    long long w = 0;
+    const double tiles = warps * parts(P.ny, 8), rows = std::min(8.0, ny), slots = 2.0 * sms;
+    const int planes = walk_planes((long long)tiles, 2LL * sms, P.nz, &w);
+    const double q = tiles * parts(P.nz, planes) * (planes + 3) / slots;
+    const double sweeps = mixed ? 167.0 + 0.97 * x + 3.74 * y + 3.93 * z : 199.0 + 2.05 * x + 5.06 * y + 3.52 * z;
+    const double tile = mixed ? w * (3.36 + 0.065 * rows) + q * (5.70 + 1.39 * rows)
+                              : w * (0.93 + 0.29 * rows) + q * (11.8 + 1.92 * rows);
+    return mixed ? sweeps < tile : 1.06 * sweeps < tile;
+}
 
 int tile3d_stage(const Tile3Args& A, cudaStream_t s, bool mixed, int& launches, LaunchMark mark, void* user) {
     const int st = mixed ? tile3_dispatch<float>(A, s) : tile3_dispatch<double>(A, s);

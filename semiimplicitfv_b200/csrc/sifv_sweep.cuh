@@ -4,12 +4,22 @@
 // divergence and the RK update stay FP64).
 //
 // Here: the parts every such kernel shares (primitive recovery, both WENO5
-// face values of a cell, the Riemann fluxes) and the 1D step: per RK stage
-// k_sweep_x (conservative -> primitive in FP64, WENO5 + Riemann flux, flux
-// divergence into an FP64 rhs buffer; a warp marches along the row, 32 cells
-// per step, neighbours exchanged by warp shuffles), then k_rk_update
-// (ExplicitSolver::step, src/ExplicitSolver.cpp:127-188).  2D and 3D run one
-// kernel per stage (sifv_march2d.cuh, sifv_tile3d.cuh).
+// face values of a cell, the Riemann fluxes), the 1D step, and the 3D step on
+// the meshes that the tiles of sifv_tile3d.cuh fit badly (sweeps_3d); 2D and
+// the other 3D meshes run one kernel per stage (sifv_march2d.cuh,
+// sifv_tile3d.cuh).  Per RK stage, one kernel per direction:
+//   x sweep  (k_sweep_x): conservative -> primitive (FP64, written back as
+//            the stage's primitive state), WENO5 + Riemann flux along x,
+//            x flux divergence; a warp marches along one row, 32 cells per
+//            step, neighbours exchanged by warp shuffles.
+//   y / z    (k_sweep_line, 3D): primitive stencil from the x sweep's output,
+//            flux divergence along y or z; each thread marches along one
+//            line segment keeping a 5-cell register window, lanes are
+//            consecutive x so every load is coalesced.
+// The z sweep adds the divergence of the earlier directions and applies the
+// SSP-RK stage update in place (ExplicitSolver::step,
+// src/ExplicitSolver.cpp:127-188); the earlier ones write / accumulate the FP64
+// rhs buffer.  In 1D k_rk_update does that after the x sweep.
 //
 // Each cell's reconstruction yields both its right-face value (from the
 // left, weno5Left) and its left-face value (from the right, weno5Right)
@@ -115,19 +125,10 @@ __device__ __forceinline__ void face_flux(int riemann, const FluxConsts& C, cons
     }
 }
 
-// Conservative -> primitive of one cell in FP64 with velocity signs of its
-// ghost mapping (1 for interior cells).
-__device__ __forceinline__ Prim5<double> load_cons_prim(const Params& P, const Fields& F, size_t src,
-                                                        const double sg[3]) {
-    double rho, u[3], p;
-    cons_to_prim_cell<0>(P, F, src, rho, u, p);
-    Prim5<double> r;
-    r.rho = rho;
-    r.u = sg[0] * u[0];
-    r.v = sg[1] * u[1];
-    r.w = sg[2] * u[2];
-    r.p = p;
-    return r;
+// Primitives of a cell of a 3D stage with the velocity signs of its ghost
+// mapping (1 for interior cells).
+__device__ __forceinline__ Prim5<double> load_prim(const Fields& F, const double* rhoP, size_t src, const double sg[3]) {
+    return Prim5<double>{rhoP[src], sg[0] * F.velU[src], sg[1] * F.velV[src], sg[2] * F.velW[src], F.pres[src]};
 }
 
 template <typename T>
@@ -145,30 +146,6 @@ __device__ __forceinline__ void recon_cell(const Prim5<T>& a, const Prim5<T>& b,
     if (DIM >= 3) weno5_pair(a.w, b.w, c.w, d.w, e.w, eps, L.w, R.w);
     else { L.w = R.w = (T)0; }
     weno5_pair(a.p, b.p, c.p, d.p, e.p, eps, L.p, R.p);
-}
-
-template <int DIM>
-__device__ __forceinline__ void rk_apply(const Fields& F, size_t c, const RKUpdate& K, double dt, double rR,
-                                         double rU, double rV, double rW, double rE) {
-    const double a3 = K.a3 * dt;
-    double r = F.rho[c], ru = F.rhoU[c], re = F.rhoE[c];
-    double rv = (DIM >= 2) ? F.rhoV[c] : 0.0, rw = (DIM >= 3) ? F.rhoW[c] : 0.0;
-    if (K.save) {
-        F.rho0[c] = r; F.rhoU0[c] = ru; F.rhoE0[c] = re;
-        if (DIM >= 2) F.rhoV0[c] = rv;
-        if (DIM >= 3) F.rhoW0[c] = rw;
-        F.pres0[c] = F.pres[c];
-    }
-    double nr = K.a1 * r + a3 * rR, nu = K.a1 * ru + a3 * rU, ne = K.a1 * re + a3 * rE;
-    double nv = K.a1 * rv + a3 * rV, nw = K.a1 * rw + a3 * rW;
-    if (K.useU0) {
-        nr += K.a2 * F.rho0[c]; nu += K.a2 * F.rhoU0[c]; ne += K.a2 * F.rhoE0[c];
-        if (DIM >= 2) nv += K.a2 * F.rhoV0[c];
-        if (DIM >= 3) nw += K.a2 * F.rhoW0[c];
-    }
-    F.rho[c] = nr; F.rhoU[c] = nu; F.rhoE[c] = ne;
-    if (DIM >= 2) F.rhoV[c] = nv;
-    if (DIM >= 3) F.rhoW[c] = nw;
 }
 
 // x sweep: each warp takes one segment [x0, x0 + seg) of one row (seg = 32 m
@@ -335,17 +312,123 @@ __global__ void __launch_bounds__(128) k_sweep_x(SweepArgs A) {
     }
 }
 
+// y or z sweep: each thread marches along one line segment [s0, s0 + seg)
+// of axis DIR at fixed x = i (consecutive lanes, coalesced) keeping the
+// 5-cell window of positions q-2 .. q+2 in registers.  The primitive values
+// of position q+3 and the update inputs of cell q-1 are loaded before the
+// arithmetic of step q so their latency overlaps it.
+template <int DIR, typename T, bool LAST>
+__global__ void __launch_bounds__(128) k_sweep_line(SweepArgs A) {
+    const Params& P = A.P;
+    const Fields& F = A.F;
+    if (A.ctl->skip) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= P.nx) return;
+    const int nLine = (DIR == 1) ? P.ny : P.nz;
+    const int other = blockIdx.z;   // k for DIR == 1, j for DIR == 2
+    const int s0 = blockIdx.y * A.seg;
+    if (s0 >= nLine) return;
+    const int s1 = min(s0 + A.seg, nLine);
+    const long st = (DIR == 1) ? (long)P.nxT : (long)P.nxT * P.nyT;
+    const size_t lineBase = (DIR == 1) ? cidx(P, i, 0, other) : cidx(P, i, other, 0);
+    const int ng = (DIR == 1) ? P.ngy : P.ngz;
+    const int bcLo = P.bc[2 * DIR], bcHi = P.bc[2 * DIR + 1];
+    const T eps = (T)A.eps;
+    const double dt = A.ctl->dt;
+
+    auto loadq = [&](int q) -> Prim5<double> {
+        if (q < -ng || q >= nLine + ng) return Prim5<double>{0.0, 0.0, 0.0, 0.0, 0.0};
+        double sn, sa;
+        int s = prim_src(q, nLine, bcLo, bcHi, sn, sa);
+        double sg[3] = {1.0, 1.0, 1.0};
+        if (s != q) { sg[0] = sa; sg[1] = sa; sg[2] = sa; sg[DIR] = sn * sa; }
+        return load_prim(F, A.rhoP, lineBase + (long)s * st, sg);
+    };
+
+    Prim5<T> w0 = to_t<T>(loadq(s0 - 3)), w1 = to_t<T>(loadq(s0 - 2)), w2 = to_t<T>(loadq(s0 - 1));
+    Prim5<T> w3 = to_t<T>(loadq(s0)), w4 = to_t<T>(loadq(s0 + 1));
+    Prim5<double> ahead = loadq(s0 + 2);
+    Prim5<T> Lm;
+    Flux4<T> Fm;
+    // position s0 - 1: only its right-face value is needed
+    {
+        Prim5<T> R;
+        recon_cell<3, T>(w0, w1, w2, w3, w4, eps, Lm, R);
+    }
+    for (int q = s0; q <= s1; ++q) {
+        w0 = w1; w1 = w2; w2 = w3; w3 = w4;
+        w4 = to_t<T>(ahead);
+        ahead = loadq(q + 3);
+        // update inputs of cell q-1
+        const bool emit = q > s0;
+        const int cq = q - 1;
+        const size_t c = lineBase + (long)cq * st;
+        double pr[5] = {0, 0, 0, 0, 0}, U[5] = {0, 0, 0, 0, 0}, U0[5] = {0, 0, 0, 0, 0}, pres = 0.0;
+        if (emit) {
+#pragma unroll
+            for (int v = 0; v < 5; ++v) pr[v] = A.rhs[v][c];
+            if (LAST) {
+                U[0] = F.rho[c]; U[1] = F.rhoU[c]; U[2] = F.rhoV[c]; U[3] = F.rhoW[c]; U[4] = F.rhoE[c];
+                if (A.K.useU0) {
+                    U0[0] = F.rho0[c]; U0[1] = F.rhoU0[c]; U0[2] = F.rhoV0[c]; U0[3] = F.rhoW0[c]; U0[4] = F.rhoE0[c];
+                }
+                if (A.K.save) pres = F.pres[c];
+            }
+        }
+        Prim5<T> L, R;
+        recon_cell<3, T>(w0, w1, w2, w3, w4, eps, L, R);
+        Flux4<T> Fq;
+        face_flux<DIR, 3, T>(P.riemann, A.C, Lm, R, Fq);
+        if (emit) {
+            double ci = A.inv[DIR][cq + ng];
+            double rR = ci * ((double)Fm.mass - (double)Fq.mass) + pr[0];
+            double rU = ci * ((double)Fm.m0 - (double)Fq.m0) + pr[1];
+            double rV = ci * ((double)Fm.m1 - (double)Fq.m1) + pr[2];
+            double rW = ci * ((double)Fm.m2 - (double)Fq.m2) + pr[3];
+            double rE = ci * ((double)Fm.energy - (double)Fq.energy) + pr[4];
+            if (LAST) {
+                const RKUpdate& K = A.K;
+                if (K.save) {
+                    F.rho0[c] = U[0]; F.rhoU0[c] = U[1]; F.rhoV0[c] = U[2]; F.rhoW0[c] = U[3]; F.rhoE0[c] = U[4];
+                    F.pres0[c] = pres;
+                }
+                const double a3 = K.a3 * dt;
+                double nr = K.a1 * U[0] + a3 * rR, nu = K.a1 * U[1] + a3 * rU, ne = K.a1 * U[4] + a3 * rE;
+                double nv = K.a1 * U[2] + a3 * rV, nw = K.a1 * U[3] + a3 * rW;
+                if (K.useU0) {
+                    nr += K.a2 * U0[0]; nu += K.a2 * U0[1]; ne += K.a2 * U0[4];
+                    nv += K.a2 * U0[2]; nw += K.a2 * U0[3];
+                }
+                F.rho[c] = nr; F.rhoU[c] = nu; F.rhoV[c] = nv; F.rhoW[c] = nw; F.rhoE[c] = ne;
+            } else {
+                A.rhs[0][c] = rR; A.rhs[1][c] = rU; A.rhs[2][c] = rV; A.rhs[3][c] = rW; A.rhs[4][c] = rE;
+            }
+        }
+        Lm = L;
+        Fm = Fq;
+    }
+}
+
 // Stage update from the complete rhs buffer (1D, where the x sweep is the
 // only direction).
-template <int DIM>
 __global__ void __launch_bounds__(256) k_rk_update(SweepArgs A) {
     if (A.ctl->skip) return;
-    long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    int i, j, k;
-    if (!int_coords(A.P, t, i, j, k)) return;
-    size_t c = cidx(A.P, i, j, k);
-    rk_apply<DIM>(A.F, c, A.K, A.ctl->dt, A.rhs[0][c], A.rhs[1][c], (DIM >= 2) ? A.rhs[2][c] : 0.0,
-                  (DIM >= 3) ? A.rhs[3][c] : 0.0, A.rhs[4][c]);
+    const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (i >= A.P.nx) return;
+    const Fields& F = A.F;
+    const RKUpdate& K = A.K;
+    const size_t c = cidx(A.P, i, 0, 0);
+    const double a3 = K.a3 * A.ctl->dt;
+    const double r = F.rho[c], ru = F.rhoU[c], re = F.rhoE[c];
+    if (K.save) {
+        F.rho0[c] = r; F.rhoU0[c] = ru; F.rhoE0[c] = re;
+        F.pres0[c] = F.pres[c];
+    }
+    double nr = K.a1 * r + a3 * A.rhs[0][c], nu = K.a1 * ru + a3 * A.rhs[1][c], ne = K.a1 * re + a3 * A.rhs[4][c];
+    if (K.useU0) {
+        nr += K.a2 * F.rho0[c]; nu += K.a2 * F.rhoU0[c]; ne += K.a2 * F.rhoE0[c];
+    }
+    F.rho[c] = nr; F.rhoU[c] = nu; F.rhoE[c] = ne;
 }
 
 // End of step: primitive state of the updated cells (interior), as the

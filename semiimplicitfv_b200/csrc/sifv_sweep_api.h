@@ -30,6 +30,7 @@ struct SweepArgs {
     FluxConsts C;
     RKUpdate K;
     double eps;
+    int seg;       // cells per thread segment (line sweeps)
     int segx;      // cells per warp segment of a row (x sweep), 32 m - 2
     double* rhs[5];  // FP64 rhs buffer (rho, rhoU, rhoV, rhoW, rhoE)
     double* rhoP;    // stage primitive density: the conservative rho is updated in place by the
@@ -111,13 +112,15 @@ struct Tile3Args {
 // timing); may be null.
 typedef void (*LaunchMark)(void* user, const char* family);
 
-// One RK stage of the 1D explicit step on the fused sweep kernels
+// One RK stage of the 1D or 3D explicit step on the fused sweep kernels
 // (mixed: FP32 reconstruction / Riemann bulk).  Returns 0 on success.
 int sweep_stage(SweepArgs A, cudaStream_t s, bool mixed, int& launches, LaunchMark mark = nullptr,
                 void* user = nullptr);
 
 int tile2d_stage(const TileArgs& A, cudaStream_t s, bool mixed, int& launches, LaunchMark mark = nullptr,
                  void* user = nullptr);
+// Whether the 3D step takes less time with the sweeps than with k_tile3d.
+bool sweeps_3d(const Params& P, bool mixed, int sms);
 int tile3d_stage(const Tile3Args& A, cudaStream_t s, bool mixed, int& launches, LaunchMark mark = nullptr,
                  void* user = nullptr);
 // out[q] = in[q] over n values (2D) or the interior cells (3D), skipped when the step is (device-side loops).
