@@ -593,9 +593,9 @@ int launch_chained(sifv_ctx* c, void (*kernel)(KArgs...), dim3 grid, unsigned th
 // per iteration), and loses where many tiles have few planes (8000 x 4 x 4
 // 7.7 against 11.5, 4 x 8000 x 4 17.6 against 25.4).  With coefficients per
 // cell, twice the arrays, its one block per SM does not hide the latency of
-// device memory: it wins while they stay in L2 (96^3 41.0 -> 24.7; 112^3 is
-// even, 128^3 57.8 against 61.0, 256^3 302 against 411) or a tile holds whole
-// rows (25 x 256 x 256 59 -> 43).
+// device memory: it wins while they stay in L2 (96^3 35.7 -> 24.7; 112^3 is
+// even, 128^3 52.3 against 61.0, 256^3 299 against 411) or a tile holds whole
+// rows (25 x 256 x 256 52 -> 43).
 bool jacobi_pairs(const sifv_ctx* c, long long walk, long long blocks, bool faceCoef) {
     const long long slots = 3LL * std::max(1, c->jacSms);
     const double planes1 = (double)((blocks + slots - 1) / slots) * std::min(c->P.nz, kJacZ);
@@ -2488,7 +2488,7 @@ int sifv_pressure_solve(sifv_ctx_t* c, const double* rho, const double* rhoc2, c
         CUDA_TRY(c, cudaMemcpyAsync(dP, res, bytes, cudaMemcpyDeviceToDevice, c->stream));
     else
         k_jacobi_finish<<<blocks((long long)c->nint, kCellThreads), kCellThreads, 0, c->stream>>>(
-            c->P, res, res, dP, c->ctl, maxIter);
+            c->P, res, dP);
     LAUNCH_CHECK(c);
     if (!onDevice) CUDA_TRY(c, cudaMemcpyAsync(pressure, dP, bytes, cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));

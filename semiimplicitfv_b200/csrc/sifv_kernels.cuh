@@ -1272,8 +1272,10 @@ __device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.w
 //
 // Per iteration, k_jacobi3 against this: 256^3 214 -> 166 us, 200 x 180 x 160
 // 88 -> 72, 128^3 43 -> 27, 64^3 27.5 -> 7.3 (whose walks of 32 planes were
-// the time).  Issue slots are 63 % busy; fetched with plain loads a plane
-// ahead, the same pair took 232 at 256^3.
+// the time).  Issue slots are 54 % busy at 200^3; fetched with plain
+// loads a plane ahead, the same pair took 232 at 256^3.  With coefficients per
+// cell: 64^3 28.9 -> 10.2, 96^3 35.7 -> 24.7, but 128^3 52.3 -> 61 and 256^3 299
+// -> 411, which stay with single iterations (jacobi_pairs).
 constexpr int kJac2Y = 16;
 constexpr int kJac2Threads = 32 * (kJac2Y + 3);
 constexpr int kJac2Row = 36;   // shared row of iterate it + 1: columns -1 .. 32
@@ -1476,15 +1478,12 @@ __global__ void __launch_bounds__(kJac2Threads, 1) k_jacobi3_pair(
     block_max_to(res2, &ctl->res[it + 1]);
 }
 
-// Copy the converged Jacobi iterate (in pA or pB by parity) to dst.
-__global__ void k_jacobi_finish(Params P, const double* __restrict__ pA, const double* __restrict__ pB,
-                                double* __restrict__ dst, const Ctl* __restrict__ ctl, int maxIter) {
-    long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+// The interior of a pressure solve's result.
+__global__ void k_jacobi_finish(Params P, const double* __restrict__ src, double* __restrict__ dst) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     int i, j, k;
     if (!int_coords(P, t, i, j, k)) return;
-    int n = ctl->jacobiDone ? ctl->jacobiDone : maxIter;
-    const double* src = (n & 1) ? pB : pA;
-    size_t c = cidx(P, i, j, k);
+    const size_t c = cidx(P, i, j, k);
     dst[c] = src[c];
 }
 

@@ -253,7 +253,7 @@ int sifv_pressure_solve_noalloc(const sifv_mesh_t* mesh, int dim, int nGhost, co
     int n = done ? done : maxIter;
     const double* result = (n & 1) ? pB : pA;
     // interior cells of the result into the caller's array (ghosts untouched)
-    k_jacobi_finish<<<g, 256, 0, s>>>(P, result, result, pressure, ctl, maxIter);
+    k_jacobi_finish<<<g, 256, 0, s>>>(P, result, pressure);
     if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess)
         return nal_fail(SIFV_ERR_CUDA, "copy-out failed");
     *iters = n;

@@ -1,7 +1,8 @@
 // sifv_stage.cuh -- one SSP-RK stage of the explicit step as one kernel, in
 // the reference's operation order (ExplicitSolver::step,
-// src/ExplicitSolver.cpp:109-190), 1D and 2D (and for the fast and mixed modes
-// on 1D meshes up to a size, fused_stage).
+// src/ExplicitSolver.cpp:109-190), 1D and 2D, where it takes less time than the
+// separate kernels (stage_pays; and for the fast and mixed modes on 1D meshes
+// up to a size, fused_stage).
 //
 // A block owns a tile of cells.  It converts the tile and its three halo
 // layers to primitives in shared memory (ghost cells through the PRIM ghost

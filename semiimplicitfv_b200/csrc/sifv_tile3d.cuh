@@ -16,13 +16,15 @@
 //   F  y divergence, and the update of plane k in FP64.
 // Every z face is solved once, x faces 33/32 and y faces 9/8 times, and a
 // cell's state is read once as a cell (and from L2 as another block's halo)
-// and written once; the three dimension sweeps this replaces passed
-// primitives and an FP64 rhs through memory (56 arrays per stage, 0.9 of
-// 2.3 ms per step at 203 x 160 x 131).  Per step, RK3, sweeps -> this, FP64 /
-// mixed: 203 x 160 x 131 2.40 -> 2.29 / 1.84 -> 1.51 ms; 64^3 437 -> 179 /
-// 357 -> 127 us; 8^3 153 -> 62 / 139 -> 51 us.  It is bound by its chains
+// and written once; three dimension sweeps pass primitives and an FP64 rhs
+// through memory (56 arrays per stage) and read the mesh again for the dt.
+// Per step, RK3, sweeps -> this, FP64 / mixed: 160^3 2.42 -> 2.07 / 1.79 ->
+// 1.41 ms; 64^3 393 -> 180 / 334 -> 127 us; 8^3 153 -> 62 / 139 -> 51 us;
+// 203 x 160 x 131 2.19 -> 2.28 / 1.78 -> 1.50 ms.  It is bound by its chains
 // between the barriers: the FP64 pipe is busy 48 % of the time at two blocks
-// per SM (shared memory).
+// per SM (shared memory), and a tile costs much the same however few of its
+// rows lie in the mesh, so meshes that fit the tiles badly keep the sweeps
+// (sweeps_3d).
 #pragma once
 
 #include "sifv_sweep.cuh"
