@@ -92,23 +92,23 @@ bool ensemble_chunks(const sifv_ensemble* e, int blockSize) {
         top = std::max(top, w);
         chunks += (double)n * ((n + cells - 1) / cells);
     }
-    int byStrips = 0, byChunks = 0;   // blocks per SM
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&byStrips, k_ensemble<double, NPH, false>, blockSize, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&byChunks, k_ensemble<double, NPH, true>, blockSize, ens_smem<NPH>(blockSize));
+    // blocks per SM by the register file (asking for the occupancy would load both kernels, 2 ms of a first run)
+    const int byStrips = (NPH == 0 ? 24 : 16) / warps, byChunks = 16 / warps;
     const bool crowded = byStrips > byChunks && strips >= 0.4 * e->sms * byStrips * top;
     return chunks * (crowded ? 1.3 : 1.08) < strips;
 }
 
 template <int NPH>
 int launch_d(const sifv_ensemble* e, int blockSize) {
-    const size_t bytes = ens_smem<NPH>(blockSize);
-    if (cudaFuncSetAttribute(k_ensemble<double, NPH, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) !=
-        cudaSuccess)
-        return -1;
-    if (ensemble_chunks<NPH>(e, blockSize))
+    if (ensemble_chunks<NPH>(e, blockSize)) {
+        const size_t bytes = ens_smem<NPH>(blockSize);
+        if (cudaFuncSetAttribute(k_ensemble<double, NPH, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) !=
+            cudaSuccess)
+            return -1;
         k_ensemble<double, NPH, true><<<e->nInst, blockSize, bytes, e->stream>>>(e->A);
-    else
+    } else {
         k_ensemble<double, NPH, false><<<e->nInst, blockSize, 0, e->stream>>>(e->A);
+    }
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
