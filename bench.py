@@ -62,8 +62,8 @@ NCU_KERNEL_SOURCES = ("semiimplicitfv_b200/csrc/sifv_march2d.cuh", "semiimplicit
 # one ncu capture each of the FP64 and the mixed march kernel on a 2048² four-quadrant Riemann stage
 # (FP64 thread operations: DADD + DMUL + DFMA issued, per interior cell)
 NCU_CAPTURE = {
-    (2, "march2d"): {"sha": "3a3a32ce917b96b3", "dram_bytes_per_cell": 89.24, "fp64_inst_per_cell": 672.0},
-    (1, "march2d"): {"sha": "3a3a32ce917b96b3", "dram_bytes_per_cell": 92.59, "fp64_inst_per_cell": 46.5},
+    (2, "march2d"): {"sha": "5df841a2ed476b2b", "dram_bytes_per_cell": 89.15, "fp64_inst_per_cell": 672.0},
+    (1, "march2d"): {"sha": "5df841a2ed476b2b", "dram_bytes_per_cell": 92.63, "fp64_inst_per_cell": 46.4},
 }
 
 
