@@ -85,7 +85,10 @@ extern "C" {
 #define SIFV_PREC_FP64_FAST 2   /* FP64, fused kernels with reassociated arithmetic (FMA, shared WENO indicators) */
 /* SIFV_PREC_MIXED and SIFV_PREC_FP64_FAST run the explicit single-phase
  * WENO5 step (any dim, any Riemann solver, no IGR, no body force); other
- * configurations are rejected by sifv_create with SIFV_ERR_UNSUPPORTED. */
+ * configurations are rejected by sifv_create with SIFV_ERR_UNSUPPORTED.
+ * In 1D both run SIFV_PREC_FP64's arithmetic, bit for bit, on up to 240000
+ * cells with RKOrder > 1, where it is the faster one; beyond that, and with
+ * RKOrder 1, their own. */
 
 /* ---- field identifiers (SolutionState members) ------------------------ */
 #define SIFV_F_RHO    0
